@@ -75,21 +75,18 @@ struct SharedLd {
   __device__ static __forceinline__ float ld(const float *p) { return *p; }
 };
 
-// Flux through the lower face of cell o along runtime axis `ax` (one HLLD
+// Riemann input at the lower face of cell o along runtime axis `ax` (one HLLD
 // instance serves all three axes).  The inputs are read at w + f*NW + o + d
 // (field f, stencil offset d): m2, m1, p1 are the offsets of the stencil
 // cells -2, -1, +1 along ax; t1, t2 the +1 offsets along the transverse axes
-// ax+1 and ax+2 (mod 3).  The 7 results go to flux + (7*ax + k)*N + oo:
-// mass, momentum x/y/z (absolute components), energy, F(B_t1), F(B_t2)
-// (calc_flux_kernel<EX>, src/library/mhd_solver.inlrb:562-636).
-template <class L = GlobalLd, class S = size_t>
-__device__ __forceinline__ void face_flux(const GridParams &g, const float *__restrict__ w, S NW, int o, int ax,
-                                          int m2, int m1, int p1, int t1, int t2, int yidx, float dt,
-                                          float *__restrict__ flux, size_t N, int oo) {
+// ax+1 and ax+2 (mod 3) (calc_flux_kernel<EX>, src/library/mhd_solver.inlrb:562-636).
+template <class L, class S>
+__device__ __forceinline__ HlldIn face_input(const GridParams &g, const float *__restrict__ w, S NW, int o, int ax,
+                                             int m2, int m1, int p1, int t1, int t2, int yidx, float dt) {
   const int e1 = ax == 2 ? 0 : ax + 1, e2 = ax == 0 ? 2 : ax - 1;
   const float *rho = w, *p = w + 4 * NW;
   const float *vn = w + (1 + ax) * NW, *v1 = w + (1 + e1) * NW, *v2 = w + (1 + e2) * NW;
-  const float *bn = w + (5 + ax) * NW, *b1 = w + (5 + e1) * NW, *b2 = w + (5 + e2) * NW;
+  const float *b1 = w + (5 + e1) * NW, *b2 = w + (5 + e2) * NW;
   const int s[4] = {m2, m1, 0, p1};
   float bc1[4], bc2[4];
 #pragma unroll
@@ -132,8 +129,31 @@ __device__ __forceinline__ void face_flux(const GridParams &g, const float *__re
     in.ul += mbv;
     in.ur += mbv;
   }
+  return in;
+}
+
+// Flux through that face.  The 7 results go to flux + (7*ax + k)*N + oo: mass,
+// momentum x/y/z (absolute components), energy, F(B_t1), F(B_t2).
+template <class L = GlobalLd, class S = size_t>
+__device__ __forceinline__ void face_flux(const GridParams &g, const float *__restrict__ w, S NW, int o, int ax,
+                                          int m2, int m1, int p1, int t1, int t2, int yidx, float dt,
+                                          float *__restrict__ flux, size_t N, int oo) {
+  const int e1 = ax == 2 ? 0 : ax + 1, e2 = ax == 0 ? 2 : ax - 1;
   float f[7];
-  hlld_flux(g.gamma, L::ld(bn + o), in, f);
+#if NMHD_FAST_ARITH
+  hlld_flux_plain(g.gamma, L::ld(w + (5 + ax) * NW + o), face_input<L>(g, w, NW, o, ax, m2, m1, p1, t1, t2, yidx, dt), f);
+#else
+  const bool ok = hlld_flux_ranged(g.gamma, g.gm1, L::ld(w + (5 + ax) * NW + o),
+                                   face_input<L>(g, w, NW, o, ax, m2, m1, p1, t1, t2, yidx, dt), f);
+  if (!(ok && g.gm1_in_range)) {
+    // The plain arithmetic, on inputs read again: the opaque offset keeps the
+    // compiler from holding the first reading's values in registers.
+    int again = o;
+    asm volatile("" : "+r"(again));
+    hlld_flux_plain(g.gamma, L::ld(w + (5 + ax) * NW + again),
+                    face_input<L>(g, w, NW, again, ax, m2, m1, p1, t1, t2, yidx, dt), f);
+  }
+#endif
   float *out = flux + (size_t)(7 * ax) * N + oo;
   out[0] = f[0];
   out[(1 + ax) * N] = f[1];

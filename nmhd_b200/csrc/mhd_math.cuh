@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "rounded.cuh"
+
 namespace nmhd {
 
 // Minbee limiter: src/library/mhd_solver.inlrb:140-145.
@@ -48,8 +50,8 @@ struct HlldIn {
   float dl, dr, ul, ur, vl, vr, wl, wr, pl, pr, byl, byr, bzl, bzr;
 };
 
-__host__ __device__ __forceinline__ void hlld_flux(const float gamma, const float Bx, const HlldIn &s,
-                                          float f[7]) {
+__host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, const float Bx, const HlldIn &s,
+                                                float f[7]) {
   const float TINY = 1.0e-10f;
   const float dens_L = s.dl, dens_R = s.dr, velx_L = s.ul, velx_R = s.ur;
   const float vely_L = s.vl, vely_R = s.vr, velz_L = s.wl, velz_R = s.wr;
@@ -219,6 +221,180 @@ __host__ __device__ __forceinline__ void hlld_flux(const float gamma, const floa
   f[4] = F4 + Sss * ess - Sd * es_ - S_ * e_;
   f[5] = F5 + Sss * By_ss - Sd * bys_ - S_ * by_;
   f[6] = F6 + Sss * Bz_ss - Sd * bzs_ - S_ * bz_;
+}
+
+// The same flux, bit for bit, for operands in ordinary ranges: false (and f
+// not set) where a quotient or root would have an operand outside the ranges
+// of rounded.cuh; the caller then takes hlld_flux_plain().
+//
+// The solver is bound by instruction issue.  Against hlld_flux_plain() it
+// saves: the range tests and branches of 16 to 18 quotients and 7 roots (one
+// test at the end); a reciprocal for each quotient by the same denominator;
+// the double reciprocal of S_M and pT*; the energy, transverse momenta and, in
+// regions 0, 1, 4 and 5, the star density and Alfven speed of the side that no
+// formula reads; and the double-star state's choice of left and right operands
+// (its sums are symmetric in the two sides up to one sign).  Each replaced
+// expression rounds to the same float:
+//  - float(double(N) * (1.0 / double(den))) is RN(N / den): a quotient of two
+//    floats is at least 2^-49 (relative) away from a midpoint of two floats,
+//    and the double product is within 2^-52 of it;
+//  - float(double(p) + 0.5 * double(B2)) is RN(p + B2 / 2): the double sum is
+//    exact unless the addends' exponents differ by more than 29, and then both
+//    round to the larger addend;
+//  - 0.5 * d * v2 and 0.5 * B2 are exact in double, so adding each with a
+//    fused multiply-add rounds where the separate addition did.
+// gm1: gamma - 1 as a denominator.
+__host__ __device__ __forceinline__ bool hlld_flux_ranged(const float gamma, const Denominator &gm1, const float Bx,
+                                                          const HlldIn &s, float f[7]) {
+  const float TINY = 1.0e-10f;
+  Ranges ranges;
+  ranges.positive(s.dl);
+  ranges.positive(s.dr);
+  ranges.positive(s.pl);
+  ranges.positive(s.pr);
+  const float B2x = Bx * Bx;
+  const float B2_L = B2x + s.byl * s.byl + s.bzl * s.bzl;
+  const float B2_R = B2x + s.byr * s.byr + s.bzr * s.bzr;
+  const float gpl = gamma * s.pl, gpr = gamma * s.pr;
+  const float gpbl = gpl + B2_L, gpbr = gpr + B2_R;
+  ranges.positive(gpbl);
+  ranges.positive(gpbr);
+  const float fsig = 1.41421354f;  // sqrtf(2.0f)
+  const float disc_L = gpbl * gpbl - 4.0f * gpl * B2x, disc_R = gpbr * gpbr - 4.0f * gpr * B2x;
+  const bool roots = fminf(disc_L, disc_R) >= 0x1p-90f;
+  const float cfl = root(quotient(gpbl + root(disc_L), denominator(2.0f * s.dl)));
+  const float cfr = root(quotient(gpbr + root(disc_R), denominator(2.0f * s.dr)));
+  const float cfmax = fsig * fmaxf(cfl, cfr);
+  const float S_L = fminf(s.ul, s.ur) - cfmax;
+  const float S_R = fmaxf(s.ul, s.ur) + cfmax;
+
+  const float pT_L = fmaf(0.5f, B2_L, s.pl), pT_R = fmaf(0.5f, B2_R, s.pr);
+  const float sRv = S_R - s.ur, sLv = S_L - s.ul;
+  ranges.positive(sRv);
+  ranges.positive(-sLv);
+  const float dsR = s.dr * sRv, dsL = s.dl * sLv;
+  const float den = dsR - dsL;
+  ranges.positive(den);
+  const float SMn = sRv * (s.dr * s.ur) - sLv * (s.dl * s.ul) - pT_R + pT_L;
+  const float pTn = dsR * pT_L - dsL * pT_R + s.dl * s.dr * sRv * sLv * (s.ur - s.ul);
+  ranges.numerator(SMn);
+  ranges.numerator(pTn);
+  const Denominator dden = denominator(den);
+  const float S_M = quotient(SMn, dden), pT_s = quotient(pTn, dden);
+
+  // The side of the contact that x/t = 0 lies on.  The operands are ordered
+  // numbers here (a NaN fails the ranges), so of the fan's conditions only
+  // the ones below decide.
+  const bool left = S_L > 0.0f || S_M >= 0.0f;
+  const float d_ = left ? s.dl : s.dr, u_ = left ? s.ul : s.ur, v_ = left ? s.vl : s.vr, w_ = left ? s.wl : s.wr;
+  const float by_ = left ? s.byl : s.byr, bz_ = left ? s.bzl : s.bzr;
+  const float B2_ = left ? B2_L : B2_R, pT_ = left ? pT_L : pT_R, p_ = left ? s.pl : s.pr;
+  const float S_ = left ? S_L : S_R, sv_ = left ? sLv : sRv, dsv_ = left ? dsL : dsR;
+  const float sm_ = S_ - S_M;
+  ranges.nonzero(sm_);
+  const Denominator dsm = denominator(sm_);
+  const float ds_ = quotient(dsv_, dsm);
+  ranges.positive(ds_);
+  const float sd_ = root(ds_);
+  const float aBx = fabsf(Bx);
+  ranges.numerator(aBx);
+  const float alf = quotient(aBx, denominator(sd_));
+  const float Ss_ = left ? S_M - alf : S_M + alf;
+
+  const float v2_ = u_ * u_ + v_ * v_ + w_ * w_;
+  const float e_ =
+      (float)fma(0.5, (double)B2_, fma(0.5, (double)d_ * (double)v2_, (double)quotient(p_, gm1)));
+  const float vB_ = u_ * Bx + v_ * by_ + w_ * bz_;
+  const float mx_ = d_ * u_, my_ = d_ * v_, mz_ = d_ * w_;
+  const float Bby = Bx * by_, Bbz = Bx * bz_;
+  f[0] = mx_;
+  f[1] = mx_ * u_ + pT_ - B2x;
+  f[2] = my_ * u_ - Bby;
+  f[3] = mz_ * u_ - Bbz;
+  f[4] = e_ * u_ + pT_ * u_ - Bx * vB_;
+  f[5] = by_ * u_ - Bx * v_;
+  f[6] = bz_ * u_ - Bx * w_;
+  const bool outer = left ? S_L > 0.0f : (Ss_ < 0.0f && S_R < 0.0f);  // regions 0 and 5
+  if (!outer) {
+    const float dn_ = dsv_ * sm_ - B2x + TINY;
+    ranges.nonzero(dn_);
+    const float q_ = d_ * (sv_ * sv_) - B2x, gap = S_M - u_;
+    const float n1 = Bby * gap, n2 = Bbz * gap, n3 = by_ * q_, n4 = bz_ * q_;
+    ranges.numerator(n1);
+    ranges.numerator(n2);
+    ranges.numerator(n3);
+    ranges.numerator(n4);
+    const Denominator ddn = denominator(dn_);
+    const float vs_ = v_ - quotient(n1, ddn), ws_ = w_ - quotient(n2, ddn);
+    const float bys_ = quotient(n3, ddn), bzs_ = quotient(n4, ddn);
+    const float vBs_ = S_M * Bx + vs_ * bys_ + ws_ * bzs_;
+    const float esn = sv_ * e_ - pT_ * u_ + pT_s * S_M + Bx * (vB_ - vBs_);
+    ranges.numerator(esn);
+    const float es_ = quotient(esn, dsm);
+    const float Us1 = ds_ * S_M, Us2 = ds_ * vs_, Us3 = ds_ * ws_;
+    if (left ? Ss_ >= 0.0f : Ss_ < 0.0f) {  // regions 1 and 4
+      f[0] = f[0] + S_ * ds_ - S_ * d_;
+      f[1] = f[1] + S_ * Us1 - S_ * mx_;
+      f[2] = f[2] + S_ * Us2 - S_ * my_;
+      f[3] = f[3] + S_ * Us3 - S_ * mz_;
+      f[4] = f[4] + S_ * es_ - S_ * e_;
+      f[5] = f[5] + S_ * bys_ - S_ * by_;
+      f[6] = f[6] + S_ * bzs_ - S_ * bz_;
+    } else {  // regions 2 and 3: the other side's star state too
+      const float Sd = Ss_ - S_;
+      f[0] = f[0] + Ss_ * ds_ - Sd * ds_ - S_ * d_;
+      f[1] = f[1] + Ss_ * Us1 - Sd * Us1 - S_ * mx_;
+      const float uo = left ? s.ur : s.ul, vo = left ? s.vr : s.vl, wo = left ? s.wr : s.wl;
+      const float byo = left ? s.byr : s.byl, bzo = left ? s.bzr : s.bzl;
+      const float svo = left ? sRv : sLv, dsvo = left ? dsR : dsL;
+      const float smo = (left ? S_R : S_L) - S_M;
+      ranges.nonzero(smo);
+      const float dso = quotient(dsvo, denominator(smo));
+      ranges.positive(dso);
+      const float sdo = root(dso);
+      const float dno = dsvo * smo - B2x + TINY;
+      ranges.nonzero(dno);
+      const float qo = (left ? s.dr : s.dl) * (svo * svo) - B2x, gapo = S_M - uo;
+      const float o1 = Bx * byo * gapo, o2 = Bx * bzo * gapo, o3 = byo * qo, o4 = bzo * qo;
+      ranges.numerator(o1);
+      ranges.numerator(o2);
+      ranges.numerator(o3);
+      ranges.numerator(o4);
+      const Denominator ddo = denominator(dno);
+      const float vso = vo - quotient(o1, ddo), wso = wo - quotient(o2, ddo);
+      const float byso = quotient(o3, ddo), bzso = quotient(o4, ddo);
+      // sign(Bx), turned for the right side: the differences below are taken
+      // from this side to the other
+      float sg = Bx != 0.0f ? copysignf(1.0f, Bx) : 0.0f;
+      sg = left ? sg : -sg;
+      const float fr = inverse(sd_ + sdo);
+      const float vely_ss = fr * (sd_ * vs_ + sdo * vso + (byso - bys_) * sg);
+      const float velz_ss = fr * (sd_ * ws_ + sdo * wso + (bzso - bzs_) * sg);
+      const float sdLR = root(ds_ * dso);
+      const float By_ss = fr * (sd_ * byso + sdo * bys_ + sdLR * (vso - vs_) * sg);
+      const float Bz_ss = fr * (sd_ * bzso + sdo * bzs_ + sdLR * (wso - ws_) * sg);
+      const float vB_ss = S_M * Bx + vely_ss * By_ss + velz_ss * Bz_ss;
+      const float ess = es_ - sd_ * (vBs_ - vB_ss) * sg;
+      f[2] = f[2] + Ss_ * (ds_ * vely_ss) - Sd * Us2 - S_ * my_;
+      f[3] = f[3] + Ss_ * (ds_ * velz_ss) - Sd * Us3 - S_ * mz_;
+      f[4] = f[4] + Ss_ * ess - Sd * es_ - S_ * e_;
+      f[5] = f[5] + Ss_ * By_ss - Sd * bys_ - S_ * by_;
+      f[6] = f[6] + Ss_ * Bz_ss - Sd * bzs_ - S_ * bz_;
+    }
+  }
+  return roots && ranges.hold();
+}
+
+// gamma - 1 as a denominator of hlld_flux_ranged(), and whether it is in range.
+__host__ __device__ __forceinline__ bool gamma_in_range(float gamma) {
+  return gamma - 1.0f >= 0x1p-40f && gamma - 1.0f <= 0x1p30f;
+}
+
+__host__ __device__ __forceinline__ void hlld_flux(const float gamma, const float Bx, const HlldIn &s, float f[7]) {
+#if !NMHD_FAST_ARITH
+  if (gamma_in_range(gamma) && hlld_flux_ranged(gamma, denominator(gamma - 1.0f), Bx, s, f)) return;
+#endif
+  hlld_flux_plain(gamma, Bx, s, f);
 }
 
 }  // namespace nmhd

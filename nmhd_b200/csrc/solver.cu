@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/nmhd.h"
+#include "mhd_math.cuh"
 #include "solver_impl.h"
 #include "step.cuh"
 
@@ -80,6 +81,9 @@ GridParams nmhd::derive_grid(const nmhd_config &c) {
   g.extent_x = comp[0];
   g.corner_y = -comp[1] / 2.0f;
   g.gamma = c.gamma;
+  volatile float gm1 = c.gamma - 1.0f;
+  g.gm1_in_range = nmhd::gamma_in_range(c.gamma);
+  g.gm1 = nmhd::denominator(gm1);
   g.cfl = c.cfl;
   g.q = c.q;
   g.omega = c.omega;

@@ -6,6 +6,7 @@
 #include <string>
 
 #include "../../include/nmhd.h"
+#include "rounded.cuh"
 
 namespace nmhd {
 
@@ -26,6 +27,8 @@ struct GridParams {
   // x / d == x * (1/d) exactly and kernels may multiply instead of divide.
   float inv_dx, inv_dy, inv_dz;
   int pow2_spacing;
+  Denominator gm1;   // gamma - 1 as a denominator (hlld_flux_ranged)
+  int gm1_in_range;  // whether it may be one
 };
 
 // Device-resident step control.  The time step is a pure function of

@@ -21,6 +21,19 @@ void cellh_hlld_many_f32(float gamma, const float *bx, const float *lr, float *o
   for (long i = 0; i < n; ++i) cellh_hlld_f32(gamma, bx[i], lr + 14 * i, out + 7 * i);
 }
 
+// hlld_flux_ranged alone: ok[i] says whether it took the state; and the plain
+// arithmetic it stands in for.
+void cellh_hlld_ranged_f32(float gamma, const float *bx, const float *lr, float *ranged, float *plain, int *ok, long n) {
+  const nmhd::Denominator gm1 = nmhd::denominator(gamma - 1.0f);
+  for (long i = 0; i < n; ++i) {
+    nmhd::HlldIn in;
+    float *dst = &in.dl;
+    for (int k = 0; k < 14; ++k) dst[k] = lr[14 * i + k];
+    ok[i] = nmhd::hlld_flux_ranged(gamma, gm1, bx[i], in, ranged + 7 * i);
+    nmhd::hlld_flux_plain(gamma, bx[i], in, plain + 7 * i);
+  }
+}
+
 void cellh_reconstruct_f32(const float *x, float *lr, long n) {
   for (long i = 0; i < n; ++i) nmhd::reconstruct4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3], lr[2 * i], lr[2 * i + 1]);
 }

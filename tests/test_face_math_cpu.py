@@ -16,6 +16,7 @@ import os
 import subprocess
 
 import numpy as np
+import pytest
 
 import adcheck
 from oracle import oracle
@@ -35,6 +36,7 @@ def lib():
         P = ctypes.c_void_p
         L.cellh_hlld_many_f32.argtypes = [ctypes.c_float, P, P, P, ctypes.c_long]
         L.cellh_reconstruct_f32.argtypes = [P, P, ctypes.c_long]
+        L.cellh_hlld_ranged_f32.argtypes = [ctypes.c_float, P, P, P, P, P, ctypes.c_long]
         _lib = L
     return _lib
 
@@ -68,6 +70,40 @@ def test_device_hlld_is_bitwise_the_oracle_in_all_regions():
         assert np.array_equal(out[i].view(np.uint32), ref.view(np.uint32)), (i, bx[i], lr[i], out[i], ref)
         regions[adcheck.hlld_region(float(GAMMA), bx[i], lr[i])] += 1
     assert (regions > 50).all(), regions
+
+
+@pytest.mark.parametrize("gamma, scale", [(5.0 / 3.0, 1.0), (1.4, 1e-3), (1.001, 1e3), (2.0, 1e-9), (5.0 / 3.0, 1e7)])
+def test_ranged_hlld_is_the_plain_one_where_it_takes_the_state(gamma, scale):
+    """hlld_flux_ranged against hlld_flux_plain (the reference's operations,
+    bitwise the oracle's above), bit for bit, on states whose pressure and
+    energies are of order `scale`; and that ordinary states are taken, tiny
+    numerators, vacuum, infinities and NaN are not."""
+    rng = np.random.default_rng(5)
+    n = 200000
+    bx, lr = riemann_inputs(rng, n)
+    bx *= np.float32(np.sqrt(scale))
+    lr[:, 2:8] *= np.float32(np.sqrt(scale))
+    lr[:, 10:14] *= np.float32(np.sqrt(scale))
+    lr[:, 8:10] *= np.float32(scale)
+    quiet = np.arange(n) % 17 == 0  # nearly equal sides: small differences everywhere
+    lr[quiet, 1::2] = lr[quiet, 0::2] * (1 + rng.normal(0, 1e-7, (quiet.sum(), 7))).astype(np.float32)
+    zero = np.arange(n) % 19 == 0   # no transverse field
+    lr[zero, 10:14] = 0
+    odd = np.arange(n) < 8          # states that must be left to the plain path
+    lr[0, 0] = 0
+    lr[1, 8] = -lr[1, 8]
+    lr[2, 4] = np.nan
+    lr[3, 12] = np.inf
+    lr[4, 0] = np.nan
+    lr[5, 2] = np.inf
+    lr[6, 2:8], lr[6, 10:14], bx[6] = 0, 1e-30, 1e-15
+    bx[7] = np.nan
+    out, ref, ok = np.empty((n, 7), np.float32), np.empty((n, 7), np.float32), np.empty(n, np.int32)
+    lib().cellh_hlld_ranged_f32(gamma, bx.ctypes.data, lr.ctypes.data, out.ctypes.data, ref.ctypes.data, ok.ctypes.data, n)
+    took = ok != 0
+    assert not took[odd].any()
+    assert took.mean() > (0.99 if 1e-6 < scale < 1e6 else 0.5), took.mean()
+    assert np.array_equal(out[took].view(np.uint32), ref[took].view(np.uint32))
 
 
 def test_device_reconstruction_is_the_minbee_limiter():
