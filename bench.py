@@ -420,7 +420,10 @@ def run_gpu_arm(args):
                 winst = tv.get("warp_instructions_per_step")
                 tsrc = "profiles/traffic_%s.json (ncu capture of kernel variant %s): %s" % (
                     wl, choice["variant"], tj.get("source", ""))
-        launches_per_step = sum(k for _, k in prof.values())
+        # the step runs the margin fill and the margin CFL, which the profile
+        # times apart, as one kernel
+        margins = sum(prof[k][1] for k in ("fill_margins", "cfl_margins"))
+        launches_per_step = sum(k for _, k in prof.values()) - margins + (margins > 0)
         line = {
             "metric": "Mcell-updates/s", "value": value, "unit": "Mcell-updates/s",
             "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

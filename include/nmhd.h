@@ -168,7 +168,8 @@ const char *nmhd_last_error(const nmhd_solver *s);
  * Runs `steps` steps launching every kernel separately with CUDA events around
  * it on the solver's stream; ms_out[i] receives the mean device time per step
  * of kernel class i and launches_out[i] (may be NULL) its kernel launches per
- * step.  Returns the
+ * step (the margin fill and the margin cells' CFL times, one kernel in
+ * nmhd_proceed, are launched and counted apart here).  Returns the
  * number of classes written (at most max), or a negative nmhd_status. */
 int nmhd_profile(nmhd_solver *s, int steps, double *ms_out, double *launches_out, int max);
 /* Kernel selection (the reference picks launch shapes with its Ruby autotuner,

@@ -372,10 +372,8 @@ void prod_step(nmhd_solver *s, Workspace &w, const StepTape<float> &t, bool cfl,
   const GridParams &g = s->g;
   float *hist = cfl ? w.dt_dev : w.hist_dummy;
   float *b0 = w.parity ? t.wo : t.wf, *b1 = w.parity ? t.wf : t.wo;  // buffer 2 = t.ws
-  if (g.my > 0 || g.mz > 0) {
-    nmhd::launch_fill(g, w.ctl, b0, b1, st);
-    if (cfl) nmhd::launch_cfl_margin(g, w.ctl, b0, b1, st);
-  }
+  if (cfl) nmhd::launch_fill_cfl(g, w.ctl, b0, b1, st);
+  else nmhd::launch_fill(g, w.ctl, b0, b1, st);
   // the default kernels (variant 5), with the tensor maps of this step's
   // buffers (the tape's buffers change from step to step)
   const nmhd::EpilogueMaps *m1 = maps_for(s, w, b0, b1, t.ws, t.f1);

@@ -300,31 +300,30 @@ __global__ void __launch_bounds__(256) k_batch_fill(const BoxDesc *__restrict__ 
   }
 }
 
-// CFL time of every cell (all = 1) or of the margin cells (all = 0) of every
-// box, folded into each box's cfl_cur; lanes of a warp that belong to the same
-// box combine before one atomic.
-__global__ void __launch_bounds__(256) k_batch_cfl(const BoxDesc *__restrict__ boxes, int nb, long long total,
-                                                   int all) {
+// CFL time of every cell (kAll), or Y-margin fill and CFL times of the margin
+// cells (one pass, margin::fill_cfl_item), of every box, folded into each box's
+// cfl_cur; lanes of a warp that belong to the same box combine before one
+// atomic.
+template <bool kAll>
+__global__ void __launch_bounds__(256) k_batch_cfl(const BoxDesc *__restrict__ boxes, int nb, long long total) {
   for (long long base = (long long)blockIdx.x * blockDim.x; base < total; base += (long long)gridDim.x * blockDim.x) {
     const long long i = base + threadIdx.x;
     int b = -1;
     unsigned bits = 0x7f800000u;
     if (i < total) {
-      b = all ? find_box(nb, i, [&](int k) { return boxes[k].cell_begin; })
-              : find_box(nb, i, [&](int k) { return boxes[k].mcfl_begin; });
+      b = kAll ? find_box(nb, i, [&](int k) { return boxes[k].cell_begin; })
+               : find_box(nb, i, [&](int k) { return boxes[k].mcfl_begin; });
       const BoxDesc &d = boxes[b];
       if (!d.ctl->done) {
-        const float *w = d.ctl->parity ? d.w1 : d.w0;
-        int x, y, z;
-        if (all) {
+        float *w = d.ctl->parity ? d.w1 : d.w0;
+        if (kAll) {
           const int c = (int)(i - d.cell_begin);
-          x = c % d.g.sx;
-          y = (c / d.g.sx) % d.g.sy;
-          z = c / (d.g.sx * d.g.sy);
+          bits = __float_as_uint(
+              margin::cfl_of_cell(d.g, w, c % d.g.sx, (c / d.g.sx) % d.g.sy, c / (d.g.sx * d.g.sy)));
         } else {
-          margin::margin_cfl_cell(d.g, (int)(i - d.mcfl_begin), &x, &y, &z);
+          bits = __float_as_uint(
+              margin::fill_cfl_item(d.g, margin::shear_shift(d.g, d.ctl->time), w, (int)(i - d.mcfl_begin)));
         }
-        bits = __float_as_uint(margin::cfl_of_cell(d.g, w, x, y, z));
       }
     }
     const unsigned same = __match_any_sync(0xffffffffu, b);
@@ -503,10 +502,8 @@ void enqueue_batch_step(nmhd_batch *b) {
   using namespace nmhd;
   cudaStream_t st = b->stream;
   const int cap = 148 * 16;
-  if (b->total_fill > 0)
-    k_batch_fill<<<grid_for(b->total_fill, cap), 256, 0, st>>>(b->d_boxes, b->n, b->total_fill);
   if (b->total_mcfl > 0)
-    k_batch_cfl<<<grid_for(b->total_mcfl, cap), 256, 0, st>>>(b->d_boxes, b->n, b->total_mcfl, 0);
+    k_batch_cfl<false><<<grid_for(b->total_mcfl, cap), 256, 0, st>>>(b->d_boxes, b->n, b->total_mcfl);
   auto stage = [&](int in_sel, int out_sel, int half, int fin) {
     for (int kind = 0; kind < 3; ++kind) launch_kind(b, kind, in_sel, out_sel, half, fin);
   };
@@ -826,7 +823,7 @@ nmhd_status nmhd_batch_proceed(nmhd_batch *b, double goal_time, int64_t max_step
     const int cap = 148 * 16;
     if (b->total_fill > 0)
       nmhd::k_batch_fill<<<grid_for(b->total_fill, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_fill);
-    nmhd::k_batch_cfl<<<grid_for(b->total_cells, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_cells, 1);
+    nmhd::k_batch_cfl<true><<<grid_for(b->total_cells, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_cells);
     BATCH_CUDA(b, cudaGetLastError());
     b->cfl_ready = true;
   }
@@ -893,7 +890,7 @@ nmhd_status nmhd_batch_prepare(nmhd_batch *b, int64_t max_steps) {
 
 int nmhd_batch_launches_per_step(const nmhd_batch *b) {
   if (!b) return NMHD_ERR_INVALID_ARGUMENT;
-  int n = (b->total_fill > 0) + (b->total_mcfl > 0);
+  int n = b->total_mcfl > 0;
   for (const BatchGroup &p : b->groups) {
     const int fixed = p.fixed_tiles > 0, general = p.total_tiles > p.fixed_tiles;
     n += 2 * (b->split[0] ? fixed + general : 1);
@@ -979,7 +976,7 @@ int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_tri
   if (!b->cfl_ready) {
     if (b->total_fill > 0)
       nmhd::k_batch_fill<<<grid_for(b->total_fill, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_fill);
-    nmhd::k_batch_cfl<<<grid_for(b->total_cells, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_cells, 1);
+    nmhd::k_batch_cfl<true><<<grid_for(b->total_cells, cap), 256, 0, b->stream>>>(b->d_boxes, b->n, b->total_cells);
   }
   // The first stage's kernels (state -> fluxes -> predictor) leave the state
   // and the clocks alone, so each can be launched again and again on it.

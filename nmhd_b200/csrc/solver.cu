@@ -186,10 +186,7 @@ void enqueue_stage(nmhd_solver *s, int in_sel, int out_sel, int half, int final_
 void enqueue_step(nmhd_solver *s) {
   const GridParams &g = s->g;
   cudaStream_t st = s->stream;
-  if (g.my > 0 || g.mz > 0) {
-    nmhd::launch_fill(g, s->ctl, s->w0, s->w1, st);
-    nmhd::launch_cfl_margin(g, s->ctl, s->w0, s->w1, st);
-  }
+  nmhd::launch_fill_cfl(g, s->ctl, s->w0, s->w1, st);
   if (s->cfg.time_order == 1) {
     enqueue_stage(s, 0, 1, 0, 1, st);
   } else {
@@ -650,7 +647,8 @@ int nmhd_profile(nmhd_solver *s, int steps, double *ms_out, double *launches_out
       NMHD_CUDA(s, cudaEventElapsedTime(&ms, ev[k], ev[k + 1]));
       acc[k] += ms;
     }
-    // kernel launches of each class: fill (Y and Z margins), margin CFL, and
+    // kernel launches of each class: fill (Y and Z margins), margin CFL (two
+    // passes here, to be timed apart; enqueue_step runs them as one), and
     // per stage the flux class (variant 3: the whole chunked stage) and the
     // update class (variant 2: CT + conserved update, variants 4 and 5: the
     // two fused; the per-stage predictor refill is timed with the first

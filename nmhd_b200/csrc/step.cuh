@@ -66,6 +66,8 @@ constexpr int kFluxFields = 21;  // 3 face directions x 7 flux components
 // Launchers (all asynchronous on `stream`).
 void launch_cfl_all(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t stream);
 void launch_cfl_margin(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t stream);
+// Both of a step's margin passes, the fill and the margin cells' CFL times, in one.
+void launch_fill_cfl(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t stream);
 void launch_fill(const GridParams &g, StepCtl *ctl, float *w0, float *w1, cudaStream_t stream);
 // Margins of the RK2 predictor wp refilled at t + dt/2 (NMHD_FLAG_HALO_PER_STAGE).
 void launch_fill_predictor(const GridParams &g, StepCtl *ctl, float *wp, cudaStream_t stream);
