@@ -194,10 +194,9 @@ __global__ void __launch_bounds__(kThreads, KIND == 0   ? NMHD_BATCH_MIN_BLOCKS_
 #ifndef NMHD_BATCH_MIN_BLOCKS_EPI
 #define NMHD_BATCH_MIN_BLOCKS_EPI 5
 #endif
-template <bool kPersist>
+template <bool kPersist, bool kFinal>
 __global__ void __launch_bounds__(kThreads, NMHD_BATCH_MIN_BLOCKS_EPI)
-    k_batch_epilogue(const __grid_constant__ BatchGroup p, int tb, int te, int in_sel, int out_sel, int half,
-                     int final_stage) {
+    k_batch_epilogue(const __grid_constant__ BatchGroup p, int tb, int te, int in_sel, int out_sel, int half) {
   __shared__ cell::epi::Smem s;
   auto tile = [&](const BoxDesc &d, int t) {
     StepCtl *ctl = d.ctl;
@@ -210,14 +209,16 @@ __global__ void __launch_bounds__(kThreads, NMHD_BATCH_MIN_BLOCKS_EPI)
     int bad = 0, timed_out = 0;
     const cell::epi::EpiMaps *maps = d.maps ? &d.maps->m : nullptr;
     const int ib = pick_index(ctl, in_sel), bb = pick_index(ctl, 0);
-    const float tcfl =
-        d.g.pow2_spacing
-            ? cell::epi::tile_epilogue<true>(s, d.g, maps, ib, bb, win, wb, wo, d.flux, x0, y0, z0, dt,
-                                            final_stage != 0, &bad, &timed_out)
-            : cell::epi::tile_epilogue<false>(s, d.g, maps, ib, bb, win, wb, wo, d.flux, x0, y0, z0, dt,
-                                             final_stage != 0, &bad, &timed_out);
+    float speed[3] = {0.0f, 0.0f, 0.0f};
+    if (d.g.pow2_spacing)
+      cell::epi::tile_epilogue<true, kFinal>(s, d.g, maps, ib, bb, win, wb, wo, d.flux, x0, y0, z0, dt, &bad,
+                                             &timed_out, speed);
+    else
+      cell::epi::tile_epilogue<false, kFinal>(s, d.g, maps, ib, bb, win, wb, wo, d.flux, x0, y0, z0, dt, &bad,
+                                              &timed_out, speed);
     if (timed_out && threadIdx.x == 0) atomicOr(&ctl->status, kStatusTimeout);
-    if (final_stage) finish_tile(ctl, (unsigned)(d.tiles_x * d.tiles_y * d.tiles_z), tcfl, bad, d.dt_hist, s.red);
+    if (kFinal)
+      finish_tile_speeds(d.g, ctl, (unsigned)(d.tiles_x * d.tiles_y * d.tiles_z), speed, bad, d.dt_hist, s.red);
   };
   if (!kPersist) {
     // tiles in the reverse of the flux pass's order (grid = te - tb CTAs,
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, NMHD_BATCH_MIN_BLOCKS_SFLUX)
       return;
     }
     const int x = x0 + a, y = y0 + b, z = z0 + c;
-    if (x < g.sx && y < g.sy && z < g.sz) cell::sfx::flux_cell_staged(g, s, d.flux, a, b, c, x, y, z, dt);
+    if (x < g.sx && y < g.sy && z < g.sz) cell::sfx::flux_cell_staged(g, s.w, d.flux, a, b, c, x, y, z, dt);
   };
   if (!kPersist) {
     const int t = tb + blockIdx.x;
@@ -475,12 +476,14 @@ void launch_kind(nmhd_batch *b, int kind, int in_sel, int out_sel, int half, int
       }
       if (kind == 2) {
         if (p.fixed_tiles > 0) {
+          auto run = [&](auto kernel, int ctas) {
+            kernel<<<ctas, blk, 0, b->stream>>>(p, 0, p.fixed_tiles, in_sel, out_sel, half);
+          };
           if (b->persist_fused)
-            nmhd::k_batch_epilogue<true><<<std::min(b->ctas[3], p.fixed_tiles), blk, 0, b->stream>>>(
-                p, 0, p.fixed_tiles, in_sel, out_sel, half, fin);
+            run(fin ? nmhd::k_batch_epilogue<true, true> : nmhd::k_batch_epilogue<true, false>,
+                std::min(b->ctas[3], p.fixed_tiles));
           else
-            nmhd::k_batch_epilogue<false><<<p.fixed_tiles, blk, 0, b->stream>>>(p, 0, p.fixed_tiles, in_sel,
-                                                                                 out_sel, half, fin);
+            run(fin ? nmhd::k_batch_epilogue<false, true> : nmhd::k_batch_epilogue<false, false>, p.fixed_tiles);
         }
         if (te > tb) {
           if (b->persist[2])
@@ -661,7 +664,7 @@ nmhd_status nmhd_batch_create(const nmhd_config *cfgs, int n, nmhd_batch **out) 
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[0], nmhd::k_batch_stage<0, true, false>, nmhd::cell::kThreads, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[1], nmhd::k_batch_stage<1, true, false>, nmhd::cell::kThreads, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[2], nmhd::k_batch_stage<2, true, false>, nmhd::cell::kThreads, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], nmhd::k_batch_epilogue<true>, nmhd::cell::kThreads, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[3], nmhd::k_batch_epilogue<true, true>, nmhd::cell::kThreads, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[4], nmhd::k_batch_flux_staged<true>, nmhd::cell::kThreads, 0);
   for (int k = 0; k < 5; ++k) b->ctas[k] = sms * std::max(1, occ[k]);
   // launch groups: consecutive boxes, tiles numbered from 0 within a group,

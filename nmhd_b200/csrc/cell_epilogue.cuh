@@ -88,7 +88,7 @@ struct __align__(128) Smem {
   float edge[kEdge];
   float wbf[kWB];
   int gx[34], gy[6], gz[4];  // wrapped global offsets of x0-1+i, (y0-1+j)*Sx, (z0-1+k)*Sx*Sy
-  float red[kThreads / 32];
+  float red[3 * kThreads / 32];
   unsigned long long mbar;   // completion of the tile's tensor copies
 };
 static_assert(3 * VelBox::N >= kWB, "face B region");
@@ -258,8 +258,8 @@ __device__ __forceinline__ void corner_emfs(Smem &s, int a, int b, int c, int wa
 // New face B (ct_core()'s face sums) of the lower x-, y- or z-face of
 // tile-local cell (a, b, c), from the corner EMFs and the face's B at the
 // start of the step (wbf: that component's field at the face).
-template <bool kPow2>
-__device__ __forceinline__ float new_bx(const Smem &s, const GridParams &g, float wbf, int a, int j, int c, float dt) {
+template <bool kPow2, class Q>
+__device__ __forceinline__ float new_bx(Q &q, const Smem &s, const GridParams &g, float wbf, int a, int j, int c, float dt) {
   const float *E = s.edge;
   const int z = ZEdge::at(a, j, c), y = YEdge::at(a, j, c);
   const float XY00 = E[eXY + z], XY01 = E[eXY + z + ZEdge::DY];
@@ -267,14 +267,14 @@ __device__ __forceinline__ float new_bx(const Smem &s, const GridParams &g, floa
   const float YX00 = E[eYX + z], YX01 = E[eYX + z + ZEdge::DY];
   const float ZX00 = E[eZX + y], ZX01 = E[eZX + y + YEdge::DZ];
   float pb = 0.0f;
-  pb = pb + 0.5f * (divs<kPow2>(XY01 - XY00, g.dy, g.inv_dy) + divs<kPow2>(XZ01 - XZ00, g.dz, g.inv_dz));
-  pb = pb - divs<kPow2>(0.5f * (YX01 - YX00), g.dy, g.inv_dy);
-  pb = pb - divs<kPow2>(0.5f * (ZX01 - ZX00), g.dz, g.inv_dz);
+  pb = pb + 0.5f * (divq<kPow2>(q, XY01 - XY00, g.dy, g.inv_dy) + divq<kPow2>(q, XZ01 - XZ00, g.dz, g.inv_dz));
+  pb = pb - divq<kPow2>(q, 0.5f * (YX01 - YX00), g.dy, g.inv_dy);
+  pb = pb - divq<kPow2>(q, 0.5f * (ZX01 - ZX00), g.dz, g.inv_dz);
   return wbf + dt * pb;
 }
 
-template <bool kPow2>
-__device__ __forceinline__ float new_by(const Smem &s, const GridParams &g, float wbf, int i, int b, int c, float dt) {
+template <bool kPow2, class Q>
+__device__ __forceinline__ float new_by(Q &q, const Smem &s, const GridParams &g, float wbf, int i, int b, int c, float dt) {
   const float *E = s.edge;
   const int z = ZEdge::at(i, b, c), x = XEdge::at(i, b, c);
   const float XY00 = E[eXY + z], XY10 = E[eXY + z + 1];
@@ -282,14 +282,14 @@ __device__ __forceinline__ float new_by(const Smem &s, const GridParams &g, floa
   const float YX00 = E[eYX + z], YX10 = E[eYX + z + 1];
   const float ZY00 = E[eZY + x], ZY01 = E[eZY + x + XEdge::DZ];
   float pb = 0.0f;
-  pb = pb - divs<kPow2>(0.5f * (XY10 - XY00), g.dx, g.inv_dx);
-  pb = pb + 0.5f * (divs<kPow2>(YZ01 - YZ00, g.dz, g.inv_dz) + divs<kPow2>(YX10 - YX00, g.dx, g.inv_dx));
-  pb = pb - divs<kPow2>(0.5f * (ZY01 - ZY00), g.dz, g.inv_dz);
+  pb = pb - divq<kPow2>(q, 0.5f * (XY10 - XY00), g.dx, g.inv_dx);
+  pb = pb + 0.5f * (divq<kPow2>(q, YZ01 - YZ00, g.dz, g.inv_dz) + divq<kPow2>(q, YX10 - YX00, g.dx, g.inv_dx));
+  pb = pb - divq<kPow2>(q, 0.5f * (ZY01 - ZY00), g.dz, g.inv_dz);
   return wbf + dt * pb;
 }
 
-template <bool kPow2>
-__device__ __forceinline__ float new_bz(const Smem &s, const GridParams &g, float wbf, int i, int j, int c, float dt) {
+template <bool kPow2, class Q>
+__device__ __forceinline__ float new_bz(Q &q, const Smem &s, const GridParams &g, float wbf, int i, int j, int c, float dt) {
   const float *E = s.edge;
   const int y = YEdge::at(i, j, c), x = XEdge::at(i, j, c);
   const float XZ00 = E[eXZ + y], XZ10 = E[eXZ + y + 1];
@@ -297,80 +297,104 @@ __device__ __forceinline__ float new_bz(const Smem &s, const GridParams &g, floa
   const float ZX00 = E[eZX + y], ZX10 = E[eZX + y + 1];
   const float ZY00 = E[eZY + x], ZY10 = E[eZY + x + XEdge::DY];
   float pb = 0.0f;
-  pb = pb - divs<kPow2>(0.5f * (XZ10 - XZ00), g.dx, g.inv_dx);
-  pb = pb - divs<kPow2>(0.5f * (YZ10 - YZ00), g.dy, g.inv_dy);
-  pb = pb + 0.5f * (divs<kPow2>(ZX10 - ZX00, g.dx, g.inv_dx) + divs<kPow2>(ZY10 - ZY00, g.dy, g.inv_dy));
+  pb = pb - divq<kPow2>(q, 0.5f * (XZ10 - XZ00), g.dx, g.inv_dx);
+  pb = pb - divq<kPow2>(q, 0.5f * (YZ10 - YZ00), g.dy, g.inv_dy);
+  pb = pb + 0.5f * (divq<kPow2>(q, ZX10 - ZX00, g.dx, g.inv_dx) + divq<kPow2>(q, ZY10 - ZY00, g.dy, g.inv_dy));
   return wbf + dt * pb;
 }
 
 // New face B of the tile's faces (each thread its cell's three) and of the
 // upper halo faces (by at y0+4 and bz at z0+2 as 6 rows of 32, bx at x0+32
-// as 8 single faces), into the shared face region.
-template <bool kPow2>
-__device__ __forceinline__ void face_b(Smem &s, const GridParams &g, int a, int b, int c, int warp, int lane,
-                                       float dt) {
+// as 8 single faces), into the shared face region.  Q: the arithmetic of the
+// divisions by spacings that are no powers of two; false where it does not
+// cover an operand.
+template <bool kPow2, class Q>
+__device__ __forceinline__ bool face_b_with(Smem &s, const GridParams &g, int a, int b, int c, int warp, int lane,
+                                            float dt) {
+  Q q;
   float *F = s.vel;  // the velocities are dead once the corner EMFs exist
   const float *W = s.wbf;
   float hb = 0.0f;
   int hr = -1;
   if (warp < 2) {
     hr = fBY + BYs::at(lane, 4, warp);
-    hb = new_by<kPow2>(s, g, W[hr], lane, 4, warp, dt);
+    hb = new_by<kPow2>(q, s, g, W[hr], lane, 4, warp, dt);
   } else if (warp < 6) {
     hr = fBZ + BZs::at(lane, warp - 2, 2);
-    hb = new_bz<kPow2>(s, g, W[hr], lane, warp - 2, 2, dt);
+    hb = new_bz<kPow2>(q, s, g, W[hr], lane, warp - 2, 2, dt);
   } else if (warp == 6 && lane < 8) {
     hr = fBX + BXs::at(32, lane & 3, lane >> 2);
-    hb = new_bx<kPow2>(s, g, W[hr], 32, lane & 3, lane >> 2, dt);
+    hb = new_bx<kPow2>(q, s, g, W[hr], 32, lane & 3, lane >> 2, dt);
   }
   const int ix = fBX + BXs::at(a, b, c), iy = fBY + BYs::at(a, b, c), iz = fBZ + BZs::at(a, b, c);
-  F[ix] = new_bx<kPow2>(s, g, W[ix], a, b, c, dt);
-  F[iy] = new_by<kPow2>(s, g, W[iy], a, b, c, dt);
-  F[iz] = new_bz<kPow2>(s, g, W[iz], a, b, c, dt);
+  F[ix] = new_bx<kPow2>(q, s, g, W[ix], a, b, c, dt);
+  F[iy] = new_by<kPow2>(q, s, g, W[iy], a, b, c, dt);
+  F[iz] = new_bz<kPow2>(q, s, g, W[iz], a, b, c, dt);
   if (hr >= 0) F[hr] = hb;
+  return q.hold();
+}
+
+template <bool kPow2>
+__device__ __forceinline__ void face_b(Smem &s, const GridParams &g, int a, int b, int c, int warp, int lane,
+                                       float dt) {
+  if (kPow2) {
+    face_b_with<true, Ieee>(s, g, a, b, c, warp, lane, dt);
+  } else if (!(face_b_with<false, Ranged>(s, g, a, b, c, warp, lane, dt) && g.ranged)) {
+    face_b_with<false, Ieee>(s, g, a, b, c, warp, lane, dt);
+  }
 }
 
 // The rest of the stage for tile-local cell (a, b, c) at global (x, y, z),
 // offset o: prim_cell() with the new face B taken from shared memory, and the
-// new B of the cell's lower faces written with the other fields.
-template <bool kPow2>
-__device__ __forceinline__ float finish_cell(const Smem &s, const GridParams &g, const float *__restrict__ wb,
-                                             float *__restrict__ wo, const float *__restrict__ flux, int a, int b,
-                                             int c, int x, int y, int z, float dt, bool final_stage, int *bad) {
+// new B of the cell's lower faces written with the other fields.  speed: the
+// largest of each axis' |v + c| and the cell's (final stage, no margin cell).
+// Q: the arithmetic of the quotients (four by the density, one by gamma - 1,
+// fifteen by the spacings where they are no powers of two, and in the final
+// stage another and a root); false where it does not cover an operand.
+template <bool kPow2, bool kFinal, class Q>
+__device__ __forceinline__ bool finish_cell_with(const Smem &s, const GridParams &g, const float *__restrict__ wb,
+                                                 float *__restrict__ wo, const float *__restrict__ flux, int a, int b,
+                                                 int c, int x, int y, int z, float dt, int *bad, float speed[3]) {
+  Q q;
+  // fields at uniform bases, cells at 32-bit byte offsets (at most 2^28 cells)
   const size_t N = (size_t)g.n;
-  const int o = (z * g.sy + y) * g.sx + x;
-  const int xp = x + 1 < g.sx ? 1 : 1 - g.sx;
-  const int yp = (y + 1 < g.sy ? 1 : 1 - g.sy) * g.sx;
-  const int zp = (z + 1 < g.sz ? 1 : 1 - g.sz) * g.sx * g.sy;
-  const float *Fx = flux, *Fy = flux + 7 * N, *Fz = flux + 14 * N;
+  const unsigned o = 4u * (unsigned)((z * g.sy + y) * g.sx + x);
+  const unsigned oxp = o + 4u * (unsigned)(x + 1 < g.sx ? 1 : 1 - g.sx);
+  const unsigned oyp = o + 4u * (unsigned)((y + 1 < g.sy ? 1 : 1 - g.sy) * g.sx);
+  const unsigned ozp = o + 4u * (unsigned)((z + 1 < g.sz ? 1 : 1 - g.sz) * g.sx * g.sy);
+  auto ld = [](const float *field, unsigned at) {
+    return __ldg(reinterpret_cast<const float *>(reinterpret_cast<const char *>(field) + at));
+  };
+  auto st = [&](int f, float v) { *reinterpret_cast<float *>(reinterpret_cast<char *>(wo + f * N) + o) = v; };
   float fl[5][6];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    fl[v][0] = __ldg(Fx + v * N + o);
-    fl[v][1] = __ldg(Fx + v * N + o + xp);
-    fl[v][2] = __ldg(Fy + v * N + o);
-    fl[v][3] = __ldg(Fy + v * N + o + yp);
-    fl[v][4] = __ldg(Fz + v * N + o);
-    fl[v][5] = __ldg(Fz + v * N + o + zp);
+  for (int k = 0; k < 5; ++k) {
+    const int vx = flux_field(0, k), vy = flux_field(1, k), vz = flux_field(2, k);
+    fl[vx][0] = ld(flux + k * N, o);
+    fl[vx][1] = ld(flux + k * N, oxp);
+    fl[vy][2] = ld(flux + (7 + k) * N, o);
+    fl[vy][3] = ld(flux + (7 + k) * N, oyp);
+    fl[vz][4] = ld(flux + (14 + k) * N, o);
+    fl[vz][5] = ld(flux + (14 + k) * N, ozp);
   }
   float pace[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     float pc = 0.0f;
-    pc = pc + divs<kPow2>(fl[v][0] - fl[v][1], g.dx, g.inv_dx);
-    pc = pc + divs<kPow2>(fl[v][2] - fl[v][3], g.dy, g.inv_dy);
-    pc = pc + divs<kPow2>(fl[v][4] - fl[v][5], g.dz, g.inv_dz);
+    pc = pc + divq<kPow2>(q, fl[v][0] - fl[v][1], g.dx, g.inv_dx);
+    pc = pc + divq<kPow2>(q, fl[v][2] - fl[v][3], g.dy, g.inv_dy);
+    pc = pc + divq<kPow2>(q, fl[v][4] - fl[v][5], g.dz, g.inv_dz);
     pace[v] = pc;
   }
   const float gm1 = g.gamma - 1.0f;
-  const float rho0 = wb[o];
-  const float vx0 = wb[N + o], vy0 = wb[2 * N + o], vz0 = wb[3 * N + o], p0 = wb[4 * N + o];
+  const float rho0 = ld(wb, o);
+  const float vx0 = ld(wb + N, o), vy0 = ld(wb + 2 * N, o), vz0 = ld(wb + 3 * N, o), p0 = ld(wb + 4 * N, o);
   const float *W = s.wbf;
   const float bxl = W[fBX + BXs::at(a, b, c)], bxh = W[fBX + BXs::at(a + 1, b, c)];
   const float byl = W[fBY + BYs::at(a, b, c)], byh = W[fBY + BYs::at(a, b + 1, c)];
   const float bzl = W[fBZ + BZs::at(a, b, c)], bzh = W[fBZ + BZs::at(a, b, c + 1)];
   const float mx0 = rho0 * vx0, my0 = rho0 * vy0, mz0 = rho0 * vz0;
-  const float e0 = p0 / gm1 + 0.5f * rho0 * (vx0 * vx0 + vy0 * vy0 + vz0 * vz0) +
+  const float e0 = q.div(p0, g.gm1) + 0.5f * rho0 * (vx0 * vx0 + vy0 * vy0 + vz0 * vz0) +
                    0.25f * (bxl * bxl + bxh * bxh + byl * byl + byh * byh + bzl * bzl + bzh * bzh);
   const float rho = rho0 + dt * pace[0];
   const float mx = mx0 + dt * pace[1];
@@ -381,8 +405,10 @@ __device__ __forceinline__ float finish_cell(const Smem &s, const GridParams &g,
   const float bx0 = Fb[fBX + BXs::at(a, b, c)], bx1 = Fb[fBX + BXs::at(a + 1, b, c)];
   const float by0 = Fb[fBY + BYs::at(a, b, c)], by1 = Fb[fBY + BYs::at(a, b + 1, c)];
   const float bz0 = Fb[fBZ + BZs::at(a, b, c)], bz1 = Fb[fBZ + BZs::at(a, b, c + 1)];
-  float vxo = mx / rho, vyo = my / rho, vzo = mz / rho;
-  const float eint = ene - 0.5f * (mx * mx + my * my + mz * mz) / rho -
+  q.positive(rho);
+  const Denominator drho = q.under(rho);
+  float vxo = q.div(mx, drho), vyo = q.div(my, drho), vzo = q.div(mz, drho);
+  const float eint = ene - q.div(0.5f * (mx * mx + my * my + mz * mz), drho) -
                      0.25f * (bx0 * bx0 + bx1 * bx1 + by0 * by0 + by1 * by1 + bz0 * bz0 + bz1 * bz1);
   const float po = eint * gm1;
   if (g.shear) {
@@ -392,40 +418,61 @@ __device__ __forceinline__ float finish_cell(const Smem &s, const GridParams &g,
     vyo = vyo + dt * ay;
     vzo = vzo + dt * 0.0f;
   }
-  wo[o] = rho;
-  wo[N + o] = vxo;
-  wo[2 * N + o] = vyo;
-  wo[3 * N + o] = vzo;
-  wo[4 * N + o] = po;
-  wo[5 * N + o] = bx0;
-  wo[6 * N + o] = by0;
-  wo[7 * N + o] = bz0;
-  float tcfl = __uint_as_float(0x7f800000u);
-  if (final_stage) {
+  st(0, rho);
+  st(1, vxo);
+  st(2, vyo);
+  st(3, vzo);
+  st(4, po);
+  st(5, bx0);
+  st(6, by0);
+  st(7, bz0);
+  if (kFinal) {
     *bad = !(rho > 0.0f) || !(po > 0.0f) || !isfinite(vxo) || !isfinite(vyo) || !isfinite(vzo) ||
            !isfinite(bx0) || !isfinite(by0) || !isfinite(bz0);
     const bool margin_cell = (y < g.my) || (y >= g.sy - g.my) || (g.mz > 0 && (z < g.mz || z >= g.sz - g.mz - 1));
     if (!margin_cell) {
+      // cfl_condition_inner/kernel (mhd_solver.inlrb:496-521); a NaN speed
+      // gives no CFL time
       const float b2 = fmaxf(bx0 * bx0, bx1 * bx1) + fmaxf(by0 * by0, by1 * by1) + fmaxf(bz0 * bz0, bz1 * bz1);
-      const float cs = sqrtf((g.gamma * po + b2) / rho);
-      tcfl = fminf(fminf(g.cfl * g.dx / fabsf(vxo + cs), g.cfl * g.dy / fabsf(vyo + cs)),
-                   g.cfl * g.dz / fabsf(vzo + cs));
+      const float c2 = q.ratio(g.gamma * po + b2, drho);
+      q.positive(c2);
+      const float cs = q.root(c2);
+      speed[0] = fmaxf(fabsf(vxo + cs), 0.0f);
+      speed[1] = fmaxf(fabsf(vyo + cs), 0.0f);
+      speed[2] = fmaxf(fabsf(vzo + cs), 0.0f);
     }
   }
-  return tcfl;
+  return q.hold();
+}
+
+template <bool kPow2, bool kFinal>
+__device__ __forceinline__ void finish_cell(const Smem &s, const GridParams &g, const float *__restrict__ wb,
+                                            float *__restrict__ wo, const float *__restrict__ flux, int a, int b,
+                                            int c, int x, int y, int z, float dt, int *bad, float speed[3]) {
+  // With power-of-two spacings only five to ten quotients are left: the range
+  // tests then cost what they save (1156 against 1147 warp instructions a
+  // stage, and a second copy of the code).
+  if (!kPow2) {
+    if (finish_cell_with<kPow2, kFinal, Ranged>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed) && g.ranged)
+      return;
+    // The compiler's division, on inputs read again (the opaque coordinate
+    // keeps the first reading's values from being held in registers).
+    asm volatile("" : "+r"(x));
+  }
+  finish_cell_with<kPow2, kFinal, Ieee>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed);
 }
 
 // The whole epilogue of one tile at (x0, y0, z0); every thread of the CTA
 // calls it.  maps: the tensor maps of these buffers (interior tiles stage by
 // tensor copies), or NULL (every tile stages with cp.async).  win: stage
 // input (velocities), wb: state at the start of the step, wo: stage output.
-// Returns the thread's CFL time (inf if none).
-template <bool kPow2>
-__device__ __forceinline__ float tile_epilogue(Smem &s, const GridParams &g, const EpiMaps *maps, int in_buf,
+// speed: the thread's largest signal speeds (unchanged where it has none).
+template <bool kPow2, bool kFinal>
+__device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, const EpiMaps *maps, int in_buf,
                                                int base_buf, const float *__restrict__ win,
                                                const float *__restrict__ wb, float *__restrict__ wo,
                                                const float *__restrict__ flux, int x0, int y0, int z0, float dt,
-                                               bool final_stage, int *bad, int *timed_out) {
+                                              int *bad, int *timed_out, float speed[3]) {
   // the thread's cell (a, b, c) of the tile, from its linear index: the same
   // for a 32 x 4 x 2 block (the single-box kernel) and a 1-D block of 256
   // threads (the batched kernel)
@@ -489,7 +536,7 @@ __device__ __forceinline__ float tile_epilogue(Smem &s, const GridParams &g, con
       mbar_wait_bounded(mb);
       __syncthreads();
       if (tid == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mb) : "memory");
-      return __uint_as_float(0x7f800000u);
+      return;
     }
     // every thread has passed the wait: the barrier's word is released
     if (tid == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mb) : "memory");
@@ -515,8 +562,7 @@ __device__ __forceinline__ float tile_epilogue(Smem &s, const GridParams &g, con
   __syncthreads();
   const int x = x0 + a, y = y0 + b, z = z0 + c;
   if (x < g.sx && y < g.sy && z < g.sz)
-    return finish_cell<kPow2>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, final_stage, bad);
-  return __uint_as_float(0x7f800000u);
+    finish_cell<kPow2, kFinal>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed);
 }
 
 }  // namespace epi

@@ -18,7 +18,7 @@ namespace {
 using namespace cell;
 
 __global__ void __launch_bounds__(kThreads, 4)
-    k_cell_flux_fast(const __grid_constant__ sfx::FluxMaps maps, GridParams g, StepCtl *ctl, const float *w0,
+    k_cell_flux_fast(const __grid_constant__ sfx::FluxMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl, const float *w0,
                      const float *w1, const float *wp, float *__restrict__ flux, int in_sel, int half) {
   __shared__ sfx::Smem s;
   if (ctl->done) return;
@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(kThreads, 4)
   }
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y, z = z0 + threadIdx.z;
   if (x < g.sx && y < g.sy && z < g.sz)
-    sfx::flux_cell_staged(g, s, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
+    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
 }
 
 }  // namespace

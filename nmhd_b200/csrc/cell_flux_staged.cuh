@@ -117,20 +117,115 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
   return true;
 }
 
-// The three lower-face fluxes of tile-local cell (a, b, c) at global (x, y,
-// z), from the staged copy: flux_cell() with shared addressing.
-__device__ __forceinline__ void flux_cell_staged(const GridParams &g, const Smem &s, float *__restrict__ flux,
-                                                 int a, int b, int c, int x, int y, int z, float dt) {
-  const size_t N = (size_t)g.n;
-  const int o = (z * g.sy + y) * g.sx + x;
-  const int ci = at(a, b, c);
-#pragma unroll 1
-  for (int ax = 0; ax < 3; ++ax) {
-    const int sa = ax == 0 ? 1 : ax == 1 ? DY : DZ;
-    const int t1 = ax == 0 ? DY : ax == 1 ? DZ : 1;
-    const int t2 = ax == 0 ? DZ : ax == 1 ? 1 : DY;
-    face_flux<SharedLd, int>(g, s.w, FS, ci, ax, -2 * sa, -sa, sa, t1, t2, y, dt, flux, N, o);
+// face_input() from the shared copy for the lower AX-face of cell index ci, in
+// the arithmetic Q.  With the axis a constant every shared read is at a
+// constant offset from the cell's address.  Transverse B is reconstructed from
+// the sums of the two faces, which halve exactly where q.slope() holds.
+template <int AX, bool kOrder2, class Q>
+__device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, const float *w, int ci, int yidx,
+                                               float half_dt) {
+  constexpr int E1 = (AX + 1) % 3, E2 = (AX + 2) % 3;
+  constexpr int stride[3] = {1, DY, DZ};
+  constexpr int sa = stride[AX], t1 = stride[E1], t2 = stride[E2];
+  const float *c = w + ci;
+  HlldIn in;
+  // density and pressure are checked to be at least 2^-40, so their slopes are
+  // 0 or far above the least and need no check
+  auto pair = [&](int f, auto &&checks, float &l, float &r) {
+    const float *p = c + f * FS;
+    if constexpr (kOrder2) reconstruct4_with(checks, p[-2 * sa], p[-sa], p[0], p[sa], l, r);
+    else l = p[-sa], r = p[0];
+  };
+  auto field = [&](int f, int t, float &l, float &r) {
+    const float *p = c + f * FS;
+    if constexpr (kOrder2)
+      reconstruct4_with(q, p[-2 * sa] + p[t - 2 * sa], p[-sa] + p[t - sa], p[0] + p[t], p[sa] + p[t + sa], l, r);
+    else
+      l = p[-sa] + p[t - sa], r = p[0] + p[t];
+    l *= 0.5f;
+    r *= 0.5f;
+  };
+  pair(0, Ieee(), in.dl, in.dr);
+  pair(1 + AX, q, in.ul, in.ur);
+  pair(1 + E1, q, in.vl, in.vr);
+  pair(1 + E2, q, in.wl, in.wr);
+  pair(4, Ieee(), in.pl, in.pr);
+  field(5 + E1, t1, in.byl, in.byr);
+  field(5 + E2, t2, in.bzl, in.bzr);
+  if (AX < 2 && g.shear) {
+    // face-centred Kepler acceleration (from v_y at x-faces, v_x at y-faces),
+    // half a stage kick on the normal velocity
+    const float *p = c + (AX == 0 ? 2 : 1) * FS;
+    const float v = 0.5f * (p[-sa] + p[0]);
+    float acc;
+    if (AX == 0) acc = -2.0f * g.omega * v;
+    else acc = 2.0f * g.omega * v + 2.0f * g.q * (g.omega * g.omega) * (g.corner_y + g.dy * ((float)yidx + 0.5f));
+    const float mbv = half_dt * acc;
+    in.ul += mbv;
+    in.ur += mbv;
   }
+  return in;
+}
+
+// The lower ax-face of cell ci in the plain arithmetic: a call, so that its
+// registers and code stay out of the loop that seldom needs it.
+static __device__ __noinline__ void plain_face(const GridParams &g, const float *w, float *flux, int ci, int ax, int o,
+                                               int yidx, float half_dt) {
+  const int sa = ax == 0 ? 1 : ax == 1 ? DY : DZ;
+  const int t1 = ax == 0 ? DY : ax == 1 ? DZ : 1, t2 = ax == 0 ? DZ : ax == 1 ? 1 : DY;
+  float f[7];
+  hlld_flux_plain(g.gamma, w[(5 + ax) * FS + ci],
+                  face_input<SharedLd>(g, w, FS, ci, ax, -2 * sa, -sa, sa, t1, t2, yidx, 2.0f * half_dt), f);
+  float *out = flux + (size_t)(7 * ax) * g.n + o;
+#pragma unroll
+  for (int k = 0; k < 7; ++k) out[(size_t)k * g.n] = f[k];
+}
+
+// The lower-face fluxes along axes ax0..ax1-1 of tile-local cell (a, b, c) at
+// global (x, y, z), from the staged copy: flux_cell()'s values.  The loop over the axes holds
+// one Riemann solver (three overflow the instruction caches) and a branch per
+// axis that reads its input: with the axis a run-time number in the input too,
+// a tenth of the instructions made addresses.  256x128x64 box: 1,912 warp
+// instructions for a warp's three faces (2,293 before), 163 us a launch (181),
+// 72 % of the issue slots filled.  Four CTAs/SM hide the start and the staging
+// of a tile better than one persistent CTA of 1,024 threads with a ring of five
+// copies (201 us: its spills miss the small L1 that is left) or a stagger of
+// the first CTAs (172 us).
+template <bool kOrder2>
+__device__ __forceinline__ void flux_cell_order(const GridParams &g, const float *w, float *__restrict__ flux, int ci,
+                                                unsigned o, int y, float dt, int ax0, int ax1) {
+  const size_t N = (size_t)g.n;
+  const float half_dt = 0.5f * dt;
+#pragma unroll 1
+  for (int ax = ax0; ax < ax1; ++ax) {
+    // field k: uniform base, 32-bit byte offset of the cell (at most 2^28 cells)
+    char *base = reinterpret_cast<char *>(flux + (size_t)(7 * ax) * N);
+    auto out = [&](int k, float v) { *reinterpret_cast<float *>(base + k * (4 * N) + 4u * o) = v; };
+#if NMHD_FAST_ARITH
+    Approximate q;
+#else
+    Ranged q;
+#endif
+    const float bn = w[(5 + ax) * FS + ci];
+    HlldIn in;
+    if (ax == 0) in = staged_input<0, kOrder2>(q, g, w, ci, y, half_dt);
+    else if (ax == 1) in = staged_input<1, kOrder2>(q, g, w, ci, y, half_dt);
+    else in = staged_input<2, kOrder2>(q, g, w, ci, y, half_dt);
+#if NMHD_FAST_ARITH
+    hlld_flux_with(q, g.gamma, Approximate::under(g.gamma - 1.0f), bn, in, out);
+#else
+    const bool ok = hlld_flux_with(q, g.gamma, g.gm1, bn, in, out);
+    if (!(ok && g.ranged)) plain_face(g, w, flux, ci, ax, (int)o, y, half_dt);
+#endif
+  }
+}
+
+__device__ __forceinline__ void flux_cell_staged(const GridParams &g, const float *w, float *__restrict__ flux,
+                                                 int a, int b, int c, int x, int y, int z, float dt, int ax0 = 0,
+                                                 int ax1 = 3) {
+  const unsigned o = (unsigned)((z * g.sy + y) * g.sx + x);
+  if (g.order2) flux_cell_order<true>(g, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
+  else flux_cell_order<false>(g, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
 }
 
 }  // namespace sfx

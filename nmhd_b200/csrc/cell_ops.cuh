@@ -50,6 +50,12 @@ __device__ __forceinline__ float divs(float x, float d, float inv) {
   return kPow2 ? x * inv : x / d;
 }
 
+// x / d for a grid spacing d with reciprocal inv, in the arithmetic Q.
+template <bool kPow2, class Q>
+__device__ __forceinline__ float divq(Q &q, float x, float d, float inv) {
+  return kPow2 ? x * inv : q.div(x, Denominator{d, inv});
+}
+
 // Time step of the current step: min(goal, CFL), clamped to the goal
 // (src/library/mhd_solver.inlrb:870-901).
 __device__ __forceinline__ float step_dt(const StepCtl *c, bool *last) {
@@ -133,36 +139,22 @@ __device__ __forceinline__ HlldIn face_input(const GridParams &g, const float *_
 }
 
 // Flux through that face.  The 7 results go to flux + (7*ax + k)*N + oo: mass,
-// momentum x/y/z (absolute components), energy, F(B_t1), F(B_t2).
+// momentum along ax, ax+1, ax+2 (mod 3), energy, F(B_t1), F(B_t2)
+// (flux_field()).
 template <class L = GlobalLd, class S = size_t>
 __device__ __forceinline__ void face_flux(const GridParams &g, const float *__restrict__ w, S NW, int o, int ax,
                                           int m2, int m1, int p1, int t1, int t2, int yidx, float dt,
                                           float *__restrict__ flux, size_t N, int oo) {
-  const int e1 = ax == 2 ? 0 : ax + 1, e2 = ax == 0 ? 2 : ax - 1;
   float f[7];
-#if NMHD_FAST_ARITH
-  hlld_flux_plain(g.gamma, L::ld(w + (5 + ax) * NW + o), face_input<L>(g, w, NW, o, ax, m2, m1, p1, t1, t2, yidx, dt), f);
-#else
-  const bool ok = hlld_flux_ranged(g.gamma, g.gm1, L::ld(w + (5 + ax) * NW + o),
-                                   face_input<L>(g, w, NW, o, ax, m2, m1, p1, t1, t2, yidx, dt), f);
-  if (!(ok && g.gm1_in_range)) {
-    // The plain arithmetic, on inputs read again: the opaque offset keeps the
-    // compiler from holding the first reading's values in registers.
-    int again = o;
-    asm volatile("" : "+r"(again));
-    hlld_flux_plain(g.gamma, L::ld(w + (5 + ax) * NW + again),
-                    face_input<L>(g, w, NW, again, ax, m2, m1, p1, t1, t2, yidx, dt), f);
-  }
-#endif
+  hlld_flux(g.gamma, L::ld(w + (5 + ax) * NW + o), face_input<L>(g, w, NW, o, ax, m2, m1, p1, t1, t2, yidx, dt), f);
   float *out = flux + (size_t)(7 * ax) * N + oo;
-  out[0] = f[0];
-  out[(1 + ax) * N] = f[1];
-  out[(1 + e1) * N] = f[2];
-  out[(1 + e2) * N] = f[3];
-  out[4 * N] = f[4];
-  out[5 * N] = f[5];
-  out[6 * N] = f[6];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) out[k * N] = f[k];
 }
+
+// Field (0 mass, 1-3 momentum x, y, z, 4 energy) in slot k < 5 of the fluxes
+// through the faces along ax.
+__host__ __device__ constexpr int flux_field(int ax, int k) { return k >= 1 && k <= 3 ? 1 + (k - 1 + ax) % 3 : k; }
 
 // The three lower-face fluxes of cell (x, y, z) (inside the box).
 __device__ __forceinline__ void flux_cell(const GridParams &g, const float *__restrict__ w,
@@ -383,17 +375,18 @@ __device__ __forceinline__ float prim_cell(const GridParams &g, const float *__r
   const int xp = x + 1 < g.sx ? 1 : 1 - g.sx;
   const int yp = (y + 1 < g.sy ? 1 : 1 - g.sy) * g.sx;
   const int zp = (z + 1 < g.sz ? 1 : 1 - g.sz) * g.sx * g.sy;
-  const float *Fx = flux, *Fy = flux + 7 * N, *Fz = flux + 14 * N;
   // all loads first: 30 face fluxes
   float fl[5][6];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    fl[v][0] = __ldg(Fx + v * N + o);
-    fl[v][1] = __ldg(Fx + v * N + o + xp);
-    fl[v][2] = __ldg(Fy + v * N + o);
-    fl[v][3] = __ldg(Fy + v * N + o + yp);
-    fl[v][4] = __ldg(Fz + v * N + o);
-    fl[v][5] = __ldg(Fz + v * N + o + zp);
+  for (int k = 0; k < 5; ++k) {
+    const float *Fx = flux + k * N, *Fy = flux + (7 + k) * N, *Fz = flux + (14 + k) * N;
+    const int vx = flux_field(0, k), vy = flux_field(1, k), vz = flux_field(2, k);
+    fl[vx][0] = __ldg(Fx + o);
+    fl[vx][1] = __ldg(Fx + o + xp);
+    fl[vy][2] = __ldg(Fy + o);
+    fl[vy][3] = __ldg(Fy + o + yp);
+    fl[vz][4] = __ldg(Fz + o);
+    fl[vz][5] = __ldg(Fz + o + zp);
   }
   float pace[5];
 #pragma unroll
@@ -468,35 +461,68 @@ __device__ __forceinline__ float block_min(float v, float *red) {
   return v;
 }
 
-// End of one tile of a final stage (called by every thread of the CTA): fold
-// the tile's CFL minimum and status into the box's control block; the last
-// of the box's `ntiles` tiles advances the box's clock (GlobalSetup::proceed,
-// mhd_solver.inlrb:981), rotates the state buffers and the CFL accumulators.
+// One thread folds a tile's CFL minimum and status into the box's control
+// block; the last of the box's `ntiles` tiles advances the box's clock
+// (GlobalSetup::proceed, mhd_solver.inlrb:981), rotates the state buffers and
+// the CFL accumulators.
+__device__ __forceinline__ void fold_tile(StepCtl *ctl, unsigned ntiles, float tcfl, int bad, float *dt_hist) {
+  atomicMin(&ctl->cfl_next, __float_as_uint(tcfl));
+  if (bad) atomicOr(&ctl->status, kStatusNumerical);
+  __threadfence();
+  const unsigned prev = atomicAdd(&ctl->blocks_done, 1u);
+  if (prev == ntiles - 1) {
+    __threadfence();
+    bool last;
+    const float dts = step_dt(ctl, &last);
+    volatile StepCtl *vc = ctl;
+    const long long gen = vc->generation;
+    dt_hist[gen % kDtHistCap] = dts;
+    vc->time = vc->time + (double)dts;
+    vc->generation = gen + 1;
+    vc->parity = vc->parity ^ 1;
+    vc->cfl_cur = atomicAdd(&ctl->cfl_next, 0u);
+    vc->cfl_next = 0x7f800000u;
+    if (!(dts >= 0.0f)) atomicOr(&ctl->status, kStatusBadDt);
+    if (last || vc->status) vc->done = 1;
+    vc->blocks_done = 0;
+  }
+}
+
+// End of one tile of a final stage (called by every thread of the CTA), from
+// the threads' CFL times.
 __device__ __forceinline__ void finish_tile(StepCtl *ctl, unsigned ntiles, float tcfl, int bad, float *dt_hist,
                                             float *red) {
   tcfl = block_min(tcfl, red);
   bad = __syncthreads_or(bad);
-  if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-    atomicMin(&ctl->cfl_next, __float_as_uint(tcfl));
-    if (bad) atomicOr(&ctl->status, kStatusNumerical);
-    __threadfence();
-    const unsigned prev = atomicAdd(&ctl->blocks_done, 1u);
-    if (prev == ntiles - 1) {
-      __threadfence();
-      bool last;
-      const float dts = step_dt(ctl, &last);
-      volatile StepCtl *vc = ctl;
-      const long long gen = vc->generation;
-      dt_hist[gen % kDtHistCap] = dts;
-      vc->time = vc->time + (double)dts;
-      vc->generation = gen + 1;
-      vc->parity = vc->parity ^ 1;
-      vc->cfl_cur = atomicAdd(&ctl->cfl_next, 0u);
-      vc->cfl_next = 0x7f800000u;
-      if (!(dts >= 0.0f)) atomicOr(&ctl->status, kStatusBadDt);
-      if (last || vc->status) vc->done = 1;
-      vc->blocks_done = 0;
+  if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) fold_tile(ctl, ntiles, tcfl, bad, dt_hist);
+}
+
+// The same from the threads' largest signal speeds |v + c| along the axes (0
+// where a cell has no CFL time).  A quotient by a larger speed never rounds to
+// a larger float, so the minimum of the cells' cfl * d / speed is the quotient
+// by the maximum: one division per axis and tile instead of three per cell,
+// and as bit patterns of non-negative floats the maxima are one instruction
+// per warp.  red: 3 * kThreads / 32 words.
+__device__ __forceinline__ void finish_tile_speeds(const GridParams &g, StepCtl *ctl, unsigned ntiles,
+                                                   const float speed[3], int bad, float *dt_hist, float *red) {
+  const int tid = (threadIdx.z * BY + threadIdx.y) * BX + threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(speed[a]));
+    if (lane == 0) red[a * (kThreads / 32) + warp] = __uint_as_float(m);
+  }
+  bad = __syncthreads_or(bad);
+  if (tid == 0) {
+    float s[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      s[a] = red[a * (kThreads / 32)];
+#pragma unroll
+      for (int w = 1; w < kThreads / 32; ++w) s[a] = fmaxf(s[a], red[a * (kThreads / 32) + w]);
     }
+    const float tcfl = fminf(fminf(g.cfl * g.dx / s[0], g.cfl * g.dy / s[1]), g.cfl * g.dz / s[2]);
+    fold_tile(ctl, ntiles, tcfl, bad, dt_hist);
   }
 }
 

@@ -43,11 +43,15 @@
 #ifndef NMHD_PRIM_MIN_BLOCKS
 #define NMHD_PRIM_MIN_BLOCKS (kPow2 ? 6 : 4)
 #endif
-// The fused epilogue holds 38.7 KB of shared memory per CTA (5 CTAs/SM).
+// The fused epilogue holds 39.4 KB of shared memory per CTA: 5 CTAs/SM (48
+// registers) with power-of-two spacings, 105 / 131 us a stage against 105 / 136
+// at 4; with other spacings its quotients spill at 48 registers, and 4 CTAs/SM
+// take 128 / 150 us where 5 take 134 / 158 (250x97x61 box).
 #ifndef NMHD_EPI_MIN_BLOCKS
-#define NMHD_EPI_MIN_BLOCKS 5
+#define NMHD_EPI_MIN_BLOCKS (kPow2 ? 5 : 4)
 #endif
-// The staged flux kernel holds 44 KB of shared memory per CTA (4 CTAs/SM).
+// The staged flux kernel holds 44 KB of shared memory per CTA: 4 CTAs/SM, 163 us
+// a launch on the 256x128x64 box (3: 165, 5: 168).
 #ifndef NMHD_SFLUX_MIN_BLOCKS
 #define NMHD_SFLUX_MIN_BLOCKS 4
 #endif
@@ -127,11 +131,11 @@ __global__ void __launch_bounds__(kThreads, NMHD_PRIM_MIN_BLOCKS) k_cell_prim(Gr
 // (variant 4); ntiles: the CTAs of this launch (the last one to finish the
 // final stage advances the clock).
 
-template <bool kPow2>
+template <bool kPow2, bool kFinal>
 __global__ void __launch_bounds__(kThreads, NMHD_EPI_MIN_BLOCKS)
-    k_cell_epilogue(const __grid_constant__ epi::EpiMaps maps, GridParams g, StepCtl *ctl, float *w0, float *w1,
-                    float *wp, const float *__restrict__ flux, float *dt_hist, int in_sel, int out_sel, int half,
-                    int final_stage, unsigned ntiles) {
+    k_cell_epilogue(const __grid_constant__ epi::EpiMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl,
+                    float *w0, float *w1, float *wp, const float *__restrict__ flux, float *dt_hist, int in_sel,
+                    int out_sel, int half, unsigned ntiles) {
   __shared__ epi::Smem s;
   if (ctl->done) return;
   float dt = step_dt(ctl, nullptr);
@@ -143,18 +147,18 @@ __global__ void __launch_bounds__(kThreads, NMHD_EPI_MIN_BLOCKS)
   // block order, so the first tiles read the fluxes written last, which are
   // still in L2
   const int tx = gridDim.x - 1 - blockIdx.x, ty = gridDim.y - 1 - blockIdx.y, tz = gridDim.z - 1 - blockIdx.z;
-  const float tcfl = epi::tile_epilogue<kPow2>(s, g, &maps, pick_index(ctl, in_sel), pick_index(ctl, 0), win, wb, wo,
-                                               flux, tx * BX, ty * BY, tz * BZ, dt, final_stage != 0, &bad,
-                                               &timed_out);
+  float speed[3] = {0.0f, 0.0f, 0.0f};
+  epi::tile_epilogue<kPow2, kFinal>(s, g, &maps, pick_index(ctl, in_sel), pick_index(ctl, 0), win, wb, wo, flux,
+                                    tx * BX, ty * BY, tz * BZ, dt, &bad, &timed_out, speed);
   if (timed_out && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0)
     atomicOr(&ctl->status, kStatusTimeout);
-  if (final_stage) finish_tile(ctl, ntiles, tcfl, bad, dt_hist, s.red);
+  if (kFinal) finish_tile_speeds(g, ctl, ntiles, speed, bad, dt_hist, s.red);
 }
 
 // Face fluxes of one stage from a shared copy of the stage input (variant
 // 5, cell_flux_staged.cuh).
 __global__ void __launch_bounds__(kThreads, NMHD_SFLUX_MIN_BLOCKS)
-    k_cell_flux_staged(const __grid_constant__ sfx::FluxMaps maps, GridParams g, StepCtl *ctl, const float *w0,
+    k_cell_flux_staged(const __grid_constant__ sfx::FluxMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl, const float *w0,
                        const float *w1, const float *wp, float *__restrict__ flux, int in_sel, int half) {
   __shared__ sfx::Smem s;
   if (ctl->done) return;
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(kThreads, NMHD_SFLUX_MIN_BLOCKS)
   }
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y, z = z0 + threadIdx.z;
   if (x < g.sx && y < g.sy && z < g.sz)
-    sfx::flux_cell_staged(g, s, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
+    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
 }
 
 dim3 cell_grid(const GridParams &g, int nz) {
@@ -277,12 +281,11 @@ void launch_cell_update_fused(const GridParams &g, StepCtl *ctl, float *w0, floa
   const unsigned ntiles = grid.x * grid.y * grid.z;
   static const EpilogueMaps kNone = {};  // enabled = 0: cp.async staging only
   const epi::EpiMaps &m = maps ? maps->m : kNone.m;
-  if (g.pow2_spacing)
-    k_cell_epilogue<true><<<grid, blk, 0, st>>>(m, g, ctl, w0, w1, wp, flux, dt_hist, in_sel, out_sel, half,
-                                                final_stage, ntiles);
-  else
-    k_cell_epilogue<false><<<grid, blk, 0, st>>>(m, g, ctl, w0, w1, wp, flux, dt_hist, in_sel, out_sel, half,
-                                                 final_stage, ntiles);
+  auto run = [&](auto kernel) {
+    kernel<<<grid, blk, 0, st>>>(m, g, ctl, w0, w1, wp, flux, dt_hist, in_sel, out_sel, half, ntiles);
+  };
+  if (g.pow2_spacing) run(final_stage ? k_cell_epilogue<true, true> : k_cell_epilogue<true, false>);
+  else run(final_stage ? k_cell_epilogue<false, true> : k_cell_epilogue<false, false>);
 }
 
 // One RK stage as a z-chunked pipeline (variant 3): chunk c of zc planes is

@@ -7,9 +7,9 @@
 // root (-prec-div=true, -prec-sqrt=true, no flush-to-zero) are the defaults.
 //
 // With NMHD_FAST_ARITH (the fast-arithmetic flux kernel, cell_fast.cu, compiled
-// with contraction and approximate division and square root) the FP64
-// sub-expressions are evaluated in float: results within the documented
-// tolerance of the reference instead of bitwise.
+// with contraction and approximate square root) hlld_flux_with<Approximate>
+// evaluates the energy in float: results within the documented tolerance of
+// the reference instead of bitwise.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -34,6 +34,37 @@ __host__ __device__ __forceinline__ void reconstruct4(float x0, float x1, float 
   const float d2 = absolute_smaller(d12, d23);
   left = x1 + d1 / 2.0f;
   right = x2 - d2 / 2.0f;
+}
+
+// The same reconstruction for slopes that are 0 or at least 2^-74 (q.slope()).
+// The limited slope is the smaller magnitude where both
+// differences have one sign, else 0: min.xorsign.abs gives the smaller
+// magnitude, positive where the signs agree, so a maximum with 0 and a sign
+// copy replace a product, two comparisons and two selections.  The product of
+// two slopes that small would underflow to 0 and switch the limiter off, which
+// is why they are left to reconstruct4(); halving a slope that is not is
+// exact, so the half slope is added in one fused multiply-add.
+template <class A>
+__host__ __device__ __forceinline__ float limited_slope(A &q, float a, float b) {
+#ifdef __CUDA_ARCH__
+  float t;
+  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t) : "f"(a), "f"(b));
+#else
+  const float m = fabsf(a) < fabsf(b) ? fabsf(a) : fabsf(b);
+  float t = (float_bits(a) ^ float_bits(b)) >> 31 ? -m : m;
+#endif
+  t = fmaxf(t, 0.0f);
+  q.slope(t);
+  return copysignf(t, b);
+}
+template <class A>
+__host__ __device__ __forceinline__ void reconstruct4_with(A &q, float x0, float x1, float x2, float x3, float &left,
+                                                           float &right) {
+  const float d01 = x1 - x0;
+  const float d12 = x2 - x1;
+  const float d23 = x3 - x2;
+  left = fmaf(0.5f, limited_slope(q, d01, d12), x1);
+  right = fmaf(-0.5f, limited_slope(q, d12, d23), x2);
 }
 
 // HLLD flux, src/library/hlld.inl:7-284 (the `#if 1` fast-magnetosonic
@@ -68,16 +99,11 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   const float B2_R = B2x + By_R * By_R + Bz_R * Bz_R;
   const float v2_R = velx_R * velx_R + vely_R * vely_R + velz_R * velz_R;
   const float gm1 = gamma - 1.0f;
-#if NMHD_FAST_ARITH
-  const float etot_L = pres_L / gm1 + 0.5f * dens_L * v2_L + 0.5f * B2_L;
-  const float etot_R = pres_R / gm1 + 0.5f * dens_R * v2_R + 0.5f * B2_R;
-#else
   // etot = p/(gamma-1) + 0.5*rho*v2 + 0.5*B2, the last two terms in double
   const float etot_L = (float)((double)(pres_L / gm1) + 0.5 * (double)dens_L * (double)v2_L +
                                0.5 * (double)B2_L);
   const float etot_R = (float)((double)(pres_R / gm1) + 0.5 * (double)dens_R * (double)v2_R +
                                0.5 * (double)B2_R);
-#endif
 
   const float gpl = gamma * pres_L, gpr = gamma * pres_R;
   const float gpbl = gpl + B2_L, gpbr = gpr + B2_R;
@@ -89,14 +115,6 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   const float S_L = fminf(velx_L, velx_R) - cfmax;
   const float S_R = fmaxf(velx_L, velx_R) + cfmax;
 
-#if NMHD_FAST_ARITH
-  const float pT_L = pres_L + 0.5f * B2_L;
-  const float pT_R = pres_R + 0.5f * B2_R;
-  const float sRv = S_R - velx_R, sLv = S_L - velx_L;
-  const float rden = 1.0f / (sRv * dens_R - sLv * dens_L);
-  const float S_M = (sRv * momx_R - sLv * momx_L - pT_R + pT_L) * rden;
-  const float pT_s = (sRv * dens_R * pT_L - sLv * dens_L * pT_R + dens_L * dens_R * sRv * sLv * (velx_R - velx_L)) * rden;
-#else
   // p + 0.5*B2: exact 0.5*B2 in double, one double add, rounded to float
   const float pT_L = (float)((double)pres_L + 0.5 * (double)B2_L);
   const float pT_R = (float)((double)pres_R + 0.5 * (double)B2_R);
@@ -109,7 +127,6 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   float pT_s = sRv * dens_R * pT_L - sLv * dens_L * pT_R;
   pT_s = pT_s + dens_L * dens_R * sRv * sLv * (velx_R - velx_L);
   pT_s = (float)((double)pT_s * rden);
-#endif
 
   const float sLm = S_L - S_M, sRm = S_R - S_M;
   // Single-star densities of both sides fix the Alfven speeds S_L*, S_R*
@@ -223,9 +240,9 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   f[6] = F6 + Sss * Bz_ss - Sd * bzs_ - S_ * bz_;
 }
 
-// The same flux, bit for bit, for operands in ordinary ranges: false (and f
-// not set) where a quotient or root would have an operand outside the ranges
-// of rounded.cuh; the caller then takes hlld_flux_plain().
+// The same flux, bit for bit, for operands in ordinary ranges: false where a
+// quotient or root has an operand outside the ranges of rounded.cuh; the
+// values are then void and the caller takes hlld_flux_plain().
 //
 // The solver is bound by instruction issue.  Against hlld_flux_plain() it
 // saves: the range tests and branches of 16 to 18 quotients and 7 roots (one
@@ -243,44 +260,54 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
 //    round to the larger addend;
 //  - 0.5 * d * v2 and 0.5 * B2 are exact in double, so adding each with a
 //    fused multiply-add rounds where the separate addition did.
-// gm1: gamma - 1 as a denominator.
-__host__ __device__ __forceinline__ bool hlld_flux_ranged(const float gamma, const Denominator &gm1, const float Bx,
-                                                          const HlldIn &s, float f[7]) {
+// gm1: gamma - 1 as a denominator.  A is the arithmetic of its quotients and
+// roots: Ranged here, Approximate (which tests no range) in the fast-arithmetic
+// kernel, where the energy's sums are in float as in the rest of that kernel.
+// out(k, v) takes flux k; it is called in each branch of the fan, where the
+// caller can store the values at once: as results of the branches they cost a
+// move each at every join.
+#ifdef __CUDA_ARCH__
+// Computes the values here, where their operands die, and not in the branch
+// that reads them.
+#define NMHD_KEEP(a, b, c, d, e) asm volatile("" : "+f"(a), "+f"(b), "+f"(c), "+f"(d), "+f"(e));
+#else
+#define NMHD_KEEP(a, b, c, d, e)
+#endif
+template <class A, class Out>
+__host__ __device__ __forceinline__ bool hlld_flux_with(A &q, const float gamma, const Denominator &gm1,
+                                                        const float Bx, const HlldIn &s, Out &&out) {
   const float TINY = 1.0e-10f;
-  Ranges ranges;
-  ranges.positive(s.dl);
-  ranges.positive(s.dr);
-  ranges.positive(s.pl);
-  ranges.positive(s.pr);
+  q.positive(s.dl);
+  q.positive(s.dr);
+  q.positive(s.pl);
+  q.positive(s.pr);
   const float B2x = Bx * Bx;
   const float B2_L = B2x + s.byl * s.byl + s.bzl * s.bzl;
   const float B2_R = B2x + s.byr * s.byr + s.bzr * s.bzr;
   const float gpl = gamma * s.pl, gpr = gamma * s.pr;
   const float gpbl = gpl + B2_L, gpbr = gpr + B2_R;
-  ranges.positive(gpbl);
-  ranges.positive(gpbr);
+  q.positive(gpbl);
+  q.positive(gpbr);
   const float fsig = 1.41421354f;  // sqrtf(2.0f)
   const float disc_L = gpbl * gpbl - 4.0f * gpl * B2x, disc_R = gpbr * gpbr - 4.0f * gpr * B2x;
   const bool roots = fminf(disc_L, disc_R) >= 0x1p-90f;
-  const float cfl = root(quotient(gpbl + root(disc_L), denominator(2.0f * s.dl)));
-  const float cfr = root(quotient(gpbr + root(disc_R), denominator(2.0f * s.dr)));
+  const float cfl = q.root(q.ratio(gpbl + q.root(disc_L), q.under(2.0f * s.dl)));
+  const float cfr = q.root(q.ratio(gpbr + q.root(disc_R), q.under(2.0f * s.dr)));
   const float cfmax = fsig * fmaxf(cfl, cfr);
   const float S_L = fminf(s.ul, s.ur) - cfmax;
   const float S_R = fmaxf(s.ul, s.ur) + cfmax;
 
   const float pT_L = fmaf(0.5f, B2_L, s.pl), pT_R = fmaf(0.5f, B2_R, s.pr);
   const float sRv = S_R - s.ur, sLv = S_L - s.ul;
-  ranges.positive(sRv);
-  ranges.positive(-sLv);
+  q.positive(sRv);
+  q.positive(-sLv);
   const float dsR = s.dr * sRv, dsL = s.dl * sLv;
   const float den = dsR - dsL;
-  ranges.positive(den);
+  q.positive(den);
   const float SMn = sRv * (s.dr * s.ur) - sLv * (s.dl * s.ul) - pT_R + pT_L;
   const float pTn = dsR * pT_L - dsL * pT_R + s.dl * s.dr * sRv * sLv * (s.ur - s.ul);
-  ranges.numerator(SMn);
-  ranges.numerator(pTn);
-  const Denominator dden = denominator(den);
-  const float S_M = quotient(SMn, dden), pT_s = quotient(pTn, dden);
+  const Denominator dden = q.under(den);
+  const float S_M = q.div_bounded(SMn, dden), pT_s = q.div_bounded(pTn, dden);
 
   // The side of the contact that x/t = 0 lies on.  The operands are ordered
   // numbers here (a NaN fails the ranges), so of the fan's conditions only
@@ -290,110 +317,107 @@ __host__ __device__ __forceinline__ bool hlld_flux_ranged(const float gamma, con
   const float by_ = left ? s.byl : s.byr, bz_ = left ? s.bzl : s.bzr;
   const float B2_ = left ? B2_L : B2_R, pT_ = left ? pT_L : pT_R, p_ = left ? s.pl : s.pr;
   const float S_ = left ? S_L : S_R, sv_ = left ? sLv : sRv, dsv_ = left ? dsL : dsR;
+  // the other side's
+  float uo = left ? s.ur : s.ul, vo = left ? s.vr : s.vl, wo = left ? s.wr : s.wl;
+  float byo = left ? s.byr : s.byl, bzo = left ? s.bzr : s.bzl;
+  float dvo = left ? s.dr : s.dl, svo = left ? sRv : sLv, dsvo = left ? dsR : dsL, So = left ? S_R : S_L;
+  NMHD_KEEP(uo, vo, wo, byo, bzo)
+  NMHD_KEEP(dvo, svo, dsvo, So, wo)
   const float sm_ = S_ - S_M;
-  ranges.nonzero(sm_);
-  const Denominator dsm = denominator(sm_);
-  const float ds_ = quotient(dsv_, dsm);
-  ranges.positive(ds_);
-  const float sd_ = root(ds_);
-  const float aBx = fabsf(Bx);
-  ranges.numerator(aBx);
-  const float alf = quotient(aBx, denominator(sd_));
+  q.positive(fabsf(sm_));
+  const Denominator dsm = q.under(sm_);
+  const float ds_ = q.ratio(dsv_, dsm);
+  q.positive(ds_);
+  const float sd_ = q.root(ds_);
+  const float alf = q.div(fabsf(Bx), q.under(sd_));
   const float Ss_ = left ? S_M - alf : S_M + alf;
 
   const float v2_ = u_ * u_ + v_ * v_ + w_ * w_;
-  const float e_ =
-      (float)fma(0.5, (double)B2_, fma(0.5, (double)d_ * (double)v2_, (double)quotient(p_, gm1)));
+  const float heat = q.ratio(p_, gm1);
+#if NMHD_FAST_ARITH
+  const float e_ = heat + 0.5f * d_ * v2_ + 0.5f * B2_;
+#else
+  const float e_ = (float)fma(0.5, (double)B2_, fma(0.5, (double)d_ * (double)v2_, (double)heat));
+#endif
   const float vB_ = u_ * Bx + v_ * by_ + w_ * bz_;
   const float mx_ = d_ * u_, my_ = d_ * v_, mz_ = d_ * w_;
   const float Bby = Bx * by_, Bbz = Bx * bz_;
-  f[0] = mx_;
-  f[1] = mx_ * u_ + pT_ - B2x;
-  f[2] = my_ * u_ - Bby;
-  f[3] = mz_ * u_ - Bbz;
-  f[4] = e_ * u_ + pT_ * u_ - Bx * vB_;
-  f[5] = by_ * u_ - Bx * v_;
-  f[6] = bz_ * u_ - Bx * w_;
-  const bool outer = left ? S_L > 0.0f : (Ss_ < 0.0f && S_R < 0.0f);  // regions 0 and 5
-  if (!outer) {
+  const float F0 = mx_;
+  const float F1 = mx_ * u_ + pT_ - B2x;
+  const float F2 = my_ * u_ - Bby;
+  const float F3 = mz_ * u_ - Bbz;
+  const float F4 = e_ * u_ + pT_ * u_ - Bx * vB_;
+  const float F5 = by_ * u_ - Bx * v_;
+  const float F6 = bz_ * u_ - Bx * w_;
+  const bool outer = left ? S_ > 0.0f : (Ss_ < 0.0f && S_ < 0.0f);  // regions 0 and 5
+  if (outer) {
+    out(0, F0), out(1, F1), out(2, F2), out(3, F3), out(4, F4), out(5, F5), out(6, F6);
+  } else {
     const float dn_ = dsv_ * sm_ - B2x + TINY;
-    ranges.nonzero(dn_);
-    const float q_ = d_ * (sv_ * sv_) - B2x, gap = S_M - u_;
-    const float n1 = Bby * gap, n2 = Bbz * gap, n3 = by_ * q_, n4 = bz_ * q_;
-    ranges.numerator(n1);
-    ranges.numerator(n2);
-    ranges.numerator(n3);
-    ranges.numerator(n4);
-    const Denominator ddn = denominator(dn_);
-    const float vs_ = v_ - quotient(n1, ddn), ws_ = w_ - quotient(n2, ddn);
-    const float bys_ = quotient(n3, ddn), bzs_ = quotient(n4, ddn);
+    q.positive(dn_);
+    const float qq = d_ * (sv_ * sv_) - B2x, gap = S_M - u_;
+    const float n1 = Bby * gap, n2 = Bbz * gap, n3 = by_ * qq, n4 = bz_ * qq;
+    const Denominator ddn = q.under(dn_);
+    const float vs_ = v_ - q.div(n1, ddn), ws_ = w_ - q.div(n2, ddn);
+    const float bys_ = q.div(n3, ddn), bzs_ = q.div(n4, ddn);
     const float vBs_ = S_M * Bx + vs_ * bys_ + ws_ * bzs_;
     const float esn = sv_ * e_ - pT_ * u_ + pT_s * S_M + Bx * (vB_ - vBs_);
-    ranges.numerator(esn);
-    const float es_ = quotient(esn, dsm);
+    const float es_ = q.div_bounded(esn, dsm);
     const float Us1 = ds_ * S_M, Us2 = ds_ * vs_, Us3 = ds_ * ws_;
     if (left ? Ss_ >= 0.0f : Ss_ < 0.0f) {  // regions 1 and 4
-      f[0] = f[0] + S_ * ds_ - S_ * d_;
-      f[1] = f[1] + S_ * Us1 - S_ * mx_;
-      f[2] = f[2] + S_ * Us2 - S_ * my_;
-      f[3] = f[3] + S_ * Us3 - S_ * mz_;
-      f[4] = f[4] + S_ * es_ - S_ * e_;
-      f[5] = f[5] + S_ * bys_ - S_ * by_;
-      f[6] = f[6] + S_ * bzs_ - S_ * bz_;
+      out(0, F0 + S_ * ds_ - S_ * d_);
+      out(1, F1 + S_ * Us1 - S_ * mx_);
+      out(2, F2 + S_ * Us2 - S_ * my_);
+      out(3, F3 + S_ * Us3 - S_ * mz_);
+      out(4, F4 + S_ * es_ - S_ * e_);
+      out(5, F5 + S_ * bys_ - S_ * by_);
+      out(6, F6 + S_ * bzs_ - S_ * bz_);
     } else {  // regions 2 and 3: the other side's star state too
       const float Sd = Ss_ - S_;
-      f[0] = f[0] + Ss_ * ds_ - Sd * ds_ - S_ * d_;
-      f[1] = f[1] + Ss_ * Us1 - Sd * Us1 - S_ * mx_;
-      const float uo = left ? s.ur : s.ul, vo = left ? s.vr : s.vl, wo = left ? s.wr : s.wl;
-      const float byo = left ? s.byr : s.byl, bzo = left ? s.bzr : s.bzl;
-      const float svo = left ? sRv : sLv, dsvo = left ? dsR : dsL;
-      const float smo = (left ? S_R : S_L) - S_M;
-      ranges.nonzero(smo);
-      const float dso = quotient(dsvo, denominator(smo));
-      ranges.positive(dso);
-      const float sdo = root(dso);
+      out(0, F0 + Ss_ * ds_ - Sd * ds_ - S_ * d_);
+      out(1, F1 + Ss_ * Us1 - Sd * Us1 - S_ * mx_);
+      const float smo = So - S_M;
+      q.positive(fabsf(smo));
+      const float dso = q.ratio(dsvo, q.under(smo));
+      q.positive(dso);
+      const float sdo = q.root(dso);
       const float dno = dsvo * smo - B2x + TINY;
-      ranges.nonzero(dno);
-      const float qo = (left ? s.dr : s.dl) * (svo * svo) - B2x, gapo = S_M - uo;
+      q.positive(dno);
+      const float qo = dvo * (svo * svo) - B2x, gapo = S_M - uo;
       const float o1 = Bx * byo * gapo, o2 = Bx * bzo * gapo, o3 = byo * qo, o4 = bzo * qo;
-      ranges.numerator(o1);
-      ranges.numerator(o2);
-      ranges.numerator(o3);
-      ranges.numerator(o4);
-      const Denominator ddo = denominator(dno);
-      const float vso = vo - quotient(o1, ddo), wso = wo - quotient(o2, ddo);
-      const float byso = quotient(o3, ddo), bzso = quotient(o4, ddo);
+      const Denominator ddo = q.under(dno);
+      const float vso = vo - q.div(o1, ddo), wso = wo - q.div(o2, ddo);
+      const float byso = q.div(o3, ddo), bzso = q.div(o4, ddo);
       // sign(Bx), turned for the right side: the differences below are taken
       // from this side to the other
       float sg = Bx != 0.0f ? copysignf(1.0f, Bx) : 0.0f;
       sg = left ? sg : -sg;
-      const float fr = inverse(sd_ + sdo);
+      const float fr = q.under(sd_ + sdo).h;
       const float vely_ss = fr * (sd_ * vs_ + sdo * vso + (byso - bys_) * sg);
       const float velz_ss = fr * (sd_ * ws_ + sdo * wso + (bzso - bzs_) * sg);
-      const float sdLR = root(ds_ * dso);
+      const float sdLR = q.root(ds_ * dso);
       const float By_ss = fr * (sd_ * byso + sdo * bys_ + sdLR * (vso - vs_) * sg);
       const float Bz_ss = fr * (sd_ * bzso + sdo * bzs_ + sdLR * (wso - ws_) * sg);
       const float vB_ss = S_M * Bx + vely_ss * By_ss + velz_ss * Bz_ss;
       const float ess = es_ - sd_ * (vBs_ - vB_ss) * sg;
-      f[2] = f[2] + Ss_ * (ds_ * vely_ss) - Sd * Us2 - S_ * my_;
-      f[3] = f[3] + Ss_ * (ds_ * velz_ss) - Sd * Us3 - S_ * mz_;
-      f[4] = f[4] + Ss_ * ess - Sd * es_ - S_ * e_;
-      f[5] = f[5] + Ss_ * By_ss - Sd * bys_ - S_ * by_;
-      f[6] = f[6] + Ss_ * Bz_ss - Sd * bzs_ - S_ * bz_;
+      out(2, F2 + Ss_ * (ds_ * vely_ss) - Sd * Us2 - S_ * my_);
+      out(3, F3 + Ss_ * (ds_ * velz_ss) - Sd * Us3 - S_ * mz_);
+      out(4, F4 + Ss_ * ess - Sd * es_ - S_ * e_);
+      out(5, F5 + Ss_ * By_ss - Sd * bys_ - S_ * by_);
+      out(6, F6 + Ss_ * Bz_ss - Sd * bzs_ - S_ * bz_);
     }
   }
-  return roots && ranges.hold();
+  return roots && q.hold();
 }
 
-// gamma - 1 as a denominator of hlld_flux_ranged(), and whether it is in range.
-__host__ __device__ __forceinline__ bool gamma_in_range(float gamma) {
-  return gamma - 1.0f >= 0x1p-40f && gamma - 1.0f <= 0x1p30f;
+__host__ __device__ __forceinline__ bool hlld_flux_ranged(const float gamma, const Denominator &gm1, const float Bx,
+                                                          const HlldIn &s, float f[7]) {
+  Ranged q;
+  return hlld_flux_with(q, gamma, gm1, Bx, s, [f](int k, float v) { f[k] = v; });
 }
 
 __host__ __device__ __forceinline__ void hlld_flux(const float gamma, const float Bx, const HlldIn &s, float f[7]) {
-#if !NMHD_FAST_ARITH
-  if (gamma_in_range(gamma) && hlld_flux_ranged(gamma, denominator(gamma - 1.0f), Bx, s, f)) return;
-#endif
+  if (denominator_in_range(gamma - 1.0f) && hlld_flux_ranged(gamma, denominator(gamma - 1.0f), Bx, s, f)) return;
   hlld_flux_plain(gamma, Bx, s, f);
 }
 

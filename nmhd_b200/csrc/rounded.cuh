@@ -21,8 +21,8 @@
 // Square root of x: from y ~ 1/sqrt(x), g = x y is corrected by y/2 times the
 // exact residual x - g^2 (Markstein, same paper).
 //
-// Ranges: |b| in [2^-40, 2^31], a = 0 or |a| in [2^-90, 2^80], x in [2^-90,
-// 2^90]; no intermediate then overflows, and no residual loses bits to
+// Ranges: |b| in [2^-40, 2^31], a = 0 or |a| >= 2^-74, |a/b| < 2^127, x in
+// [2^-90, 2^90]; no intermediate then overflows, and no residual loses bits to
 // underflow.  A zero quotient may come back as +0 where it is -0.
 #pragma once
 #include <cuda_runtime.h>
@@ -64,6 +64,8 @@ struct Denominator {
 };
 __host__ __device__ __forceinline__ Denominator denominator(float b) { return Denominator{b, inverse(b)}; }
 
+__host__ __device__ __forceinline__ bool denominator_in_range(float b) { return b >= 0x1p-40f && b <= 0x1p30f; }
+
 // RN(a/b).
 __host__ __device__ __forceinline__ float quotient(float a, const Denominator &d) {
   const float t = a * d.h;
@@ -88,31 +90,73 @@ __host__ __device__ __forceinline__ unsigned float_bits(float v) {
 }
 
 // Whether the operands seen so far lie in the ranges above, kept as extremes
-// of their bit patterns (NaN, infinities and, for positive(), negative values
-// compare above every finite bound).
+// of their bit patterns.  positive(): in [2^-40, 2^24], as the largest distance
+// above the lower bound (unsigned: smaller, negative and NaN values wrap or lie
+// far above).  tiny(): 0 or at least 2^-74, as the least pattern less one (0
+// becomes the largest).  Two accumulators and one instruction a value: more of
+// either cost the Riemann solver spills.
 struct Ranges {
-  unsigned least = 0x7fffffffu, most = 0u;  // values that must lie in [2^-40, 2^30]
-  unsigned zleast = 0xffffffffu, zmost = 0u;  // values that must be 0 or in [2^-90, 2^80]
+  static constexpr unsigned kLow = (127u - 40u) << 23, kHigh = (127u + 24u) << 23, kTiny = (127u - 74u) << 23;
+  unsigned far = 0u, least = 0xffffffffu;
   __host__ __device__ __forceinline__ void positive(float v) {
-    const unsigned u = float_bits(v);
+    const unsigned u = float_bits(v) - kLow;
+    far = u > far ? u : far;
+  }
+  __host__ __device__ __forceinline__ void tiny(float v) {  // v >= 0
+    const unsigned u = float_bits(v) - 1u;
     least = u < least ? u : least;
-    most = u > most ? u : most;
   }
-  __host__ __device__ __forceinline__ void nonzero(float v) {
-    const unsigned u = float_bits(v) & 0x7fffffffu;
-    least = u < least ? u : least;
-    most = u > most ? u : most;
+  __host__ __device__ __forceinline__ bool hold() const { return far <= kHigh - kLow && least >= kTiny - 1u; }
+};
+
+// Arithmetic of code written once over its quotients and roots: div() checks
+// its numerator (div_bounded() also from above, by 2^60), ratio() and root()
+// leave their operands to positive(), and hold() says at the end whether every
+// operand was in range.
+//
+// Ranged: the operations above, to be repeated with Ieee where hold() is false.
+struct Ranged {
+  Ranges r;
+  __host__ __device__ __forceinline__ void positive(float v) { r.positive(v); }
+  __host__ __device__ __forceinline__ void slope(float v) { r.tiny(v); }
+  __host__ __device__ __forceinline__ static Denominator under(float b) { return denominator(b); }
+  __host__ __device__ __forceinline__ static float ratio(float a, const Denominator &d) { return quotient(a, d); }
+  __host__ __device__ __forceinline__ float div(float a, const Denominator &d) {
+    r.tiny(fabsf(a));
+    return quotient(a, d);
   }
-  __host__ __device__ __forceinline__ void numerator(float v) {
-    const unsigned u = float_bits(v) << 1;
-    zmost = u > zmost ? u : zmost;
-    zleast = u - 1u < zleast ? u - 1u : zleast;  // 0 becomes the largest
+  __host__ __device__ __forceinline__ float div_bounded(float a, const Denominator &d) {
+    // |a| 2^-36 + 2^-40 <= 2^24
+    r.positive(fmaf(fabsf(a), 0x1p-36f, 0x1p-40f));
+    return div(a, d);
   }
-  __host__ __device__ __forceinline__ bool hold() const {
-    constexpr unsigned one = 127u;
-    return least >= (one - 40u) << 23 && most <= (one + 30u) << 23 && zleast >= ((one - 90u) << 24) - 1u &&
-           zmost <= (one + 80u) << 24;
-  }
+  __host__ __device__ __forceinline__ static float root(float x) { return nmhd::root(x); }
+  __host__ __device__ __forceinline__ bool hold() const { return r.hold(); }
+};
+
+// The compiler's division and square root, for any operands.
+struct Ieee {
+  __host__ __device__ __forceinline__ static void positive(float) {}
+  __host__ __device__ __forceinline__ static void slope(float) {}
+  __host__ __device__ __forceinline__ static Denominator under(float b) { return Denominator{b, 0.0f}; }
+  __host__ __device__ __forceinline__ static float ratio(float a, const Denominator &d) { return a / d.b; }
+  __host__ __device__ __forceinline__ static float div(float a, const Denominator &d) { return a / d.b; }
+  __host__ __device__ __forceinline__ static float div_bounded(float a, const Denominator &d) { return a / d.b; }
+  __host__ __device__ __forceinline__ static float root(float x) { return sqrtf(x); }
+  __host__ __device__ __forceinline__ static bool hold() { return true; }
+};
+
+// Products with approximate reciprocals (within 2 ulp), for the opt-in fast
+// arithmetic.
+struct Approximate {
+  __device__ __forceinline__ static void positive(float) {}
+  __device__ __forceinline__ static void slope(float) {}
+  __device__ __forceinline__ static Denominator under(float b) { return Denominator{b, approx_inverse(b)}; }
+  __device__ __forceinline__ static float ratio(float a, const Denominator &d) { return a * d.h; }
+  __device__ __forceinline__ static float div(float a, const Denominator &d) { return a * d.h; }
+  __device__ __forceinline__ static float div_bounded(float a, const Denominator &d) { return a * d.h; }
+  __device__ __forceinline__ static float root(float x) { return sqrtf(x); }
+  __device__ __forceinline__ static bool hold() { return true; }
 };
 
 }  // namespace nmhd

@@ -82,7 +82,6 @@ GridParams nmhd::derive_grid(const nmhd_config &c) {
   g.corner_y = -comp[1] / 2.0f;
   g.gamma = c.gamma;
   volatile float gm1 = c.gamma - 1.0f;
-  g.gm1_in_range = nmhd::gamma_in_range(c.gamma);
   g.gm1 = nmhd::denominator(gm1);
   g.cfl = c.cfl;
   g.q = c.q;
@@ -101,6 +100,8 @@ GridParams nmhd::derive_grid(const nmhd_config &c) {
   g.inv_dx = 1.0f / g.dx;
   g.inv_dy = 1.0f / g.dy;
   g.inv_dz = 1.0f / g.dz;
+  g.ranged = nmhd::denominator_in_range(gm1) && nmhd::denominator_in_range(g.dx) &&
+             nmhd::denominator_in_range(g.dy) && nmhd::denominator_in_range(g.dz);
   return g;
 }
 

@@ -27,8 +27,8 @@ struct GridParams {
   // x / d == x * (1/d) exactly and kernels may multiply instead of divide.
   float inv_dx, inv_dy, inv_dz;
   int pow2_spacing;
-  Denominator gm1;   // gamma - 1 as a denominator (hlld_flux_ranged)
-  int gm1_in_range;  // whether it may be one
+  Denominator gm1;  // gamma - 1 as a denominator
+  int ranged;       // gamma - 1 and the spacings lie in the range of denominators (rounded.cuh)
 };
 
 // Device-resident step control.  The time step is a pure function of

@@ -38,4 +38,14 @@ void cellh_reconstruct_f32(const float *x, float *lr, long n) {
   for (long i = 0; i < n; ++i) nmhd::reconstruct4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3], lr[2 * i], lr[2 * i + 1]);
 }
 
+// reconstruct4_with alone: ok[i] says whether its slopes were in range.
+void cellh_reconstruct_ranged_f32(const float *x, float *lr, int *ok, long n) {
+  for (long i = 0; i < n; ++i) {
+    nmhd::Ranged q;
+    nmhd::reconstruct4_with(q, x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3], lr[2 * i], lr[2 * i + 1]);
+    q.positive(1.0f);
+    ok[i] = q.hold();
+  }
+}
+
 }  // extern "C"
