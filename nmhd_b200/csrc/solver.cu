@@ -138,14 +138,27 @@ nmhd_status nmhd::validate_config(const nmhd_config *c, std::string &why) {
 namespace {
 
 nmhd_status read_ctl(nmhd_solver *s, StepCtl &h) {
+  if (s->ctl_known && !s->ctl_shared) {
+    h = s->mirror;
+    return NMHD_OK;
+  }
   NMHD_CUDA(s, cudaMemcpyAsync(&h, s->ctl, sizeof(StepCtl), cudaMemcpyDeviceToHost, s->stream));
   NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
+  s->mirror = h;
+  s->ctl_known = true;
   return NMHD_OK;
 }
 
+__global__ void k_write_ctl(StepCtl *ctl, StepCtl h) { *ctl = h; }
+
+// In the stream's order, without waiting: the values travel as the kernel's
+// parameter.
 nmhd_status write_ctl(nmhd_solver *s, const StepCtl &h) {
-  NMHD_CUDA(s, cudaMemcpyAsync(s->ctl, &h, sizeof(StepCtl), cudaMemcpyHostToDevice, s->stream));
-  NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
+  s->ctl_known = false;
+  k_write_ctl<<<1, 1, 0, s->stream>>>(s->ctl, h);
+  NMHD_CUDA(s, cudaGetLastError());
+  s->mirror = h;
+  s->ctl_known = true;
   return NMHD_OK;
 }
 
@@ -222,17 +235,22 @@ void drop_graphs(nmhd_solver *s) {
 
 nmhd_status copy_fields(nmhd_solver *s, float *dev_base, const float *const in[8], float *const out[8],
                         int on_device) {
-  const size_t bytes = sizeof(float) * (size_t)s->g.n;
+  const size_t n = (size_t)s->g.n;
+  // fields that lie one after another, as on the device, are one copy
+  bool together = true;
   for (int v = 0; v < 8; ++v) {
-    if (in) {
-      if (!in[v]) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
-      NMHD_CUDA(s, cudaMemcpyAsync(dev_base + (size_t)v * s->g.n, in[v], bytes,
+    const float *p = in ? in[v] : out[v], *first = in ? in[0] : out[0];
+    if (!p) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
+    together = together && p == first + v * n;
+  }
+  const size_t bytes = sizeof(float) * n * (together ? 8 : 1);
+  for (int v = 0; v < (together ? 1 : 8); ++v) {
+    if (in)
+      NMHD_CUDA(s, cudaMemcpyAsync(dev_base + v * n, in[v], bytes,
                                    on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s->stream));
-    } else {
-      if (!out[v]) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
-      NMHD_CUDA(s, cudaMemcpyAsync(out[v], dev_base + (size_t)v * s->g.n, bytes,
+    else
+      NMHD_CUDA(s, cudaMemcpyAsync(out[v], dev_base + v * n, bytes,
                                    on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s->stream));
-    }
   }
   NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
   return NMHD_OK;
@@ -403,6 +421,7 @@ nmhd_status nmhd_proceed(nmhd_solver *s, double goal_time, double wallclock_limi
   }
   st = write_ctl(s, h);
   if (st != NMHD_OK) return st;
+  s->ctl_known = false;  // until the last batch's copy is read
   if (!s->cfl_ready) {
     // CFL time of the fresh state, after its margins are filled.
     nmhd::launch_fill(s->g, s->ctl, s->w0, s->w1, s->stream);
@@ -459,6 +478,8 @@ nmhd_status nmhd_proceed(nmhd_solver *s, double goal_time, double wallclock_limi
   // a batch still in flight ran after the goal or the error: its kernels
   // returned at once and the clock read above is final
   NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
+  s->mirror = h;
+  s->ctl_known = true;
   if (steps_done) *steps_done = h.generation - gen0;
   return result;
 }
@@ -566,6 +587,7 @@ int nmhd_profile(nmhd_solver *s, int steps, double *ms_out, double *launches_out
   if (!s->cfl_ready) h.cfl_cur = h.cfl_next = 0x7f800000u;
   st = write_ctl(s, h);
   if (st != NMHD_OK) return st;
+  s->ctl_known = false;
   if (!s->cfl_ready) {
     nmhd::launch_fill(s->g, s->ctl, s->w0, s->w1, s->stream);
     nmhd::launch_cfl_all(s->g, s->ctl, s->w0, s->w1, s->stream);
@@ -771,6 +793,7 @@ int nmhd_autotune(nmhd_solver *s, int steps, double *trials_out, int max_trials)
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
   const int saved_variant = s->variant;
   const nmhd::TileShape saved_shape = s->shape;
+  s->ctl_known = false;
   double best = 1e30;
   TuneChoice choice = {saved_variant, saved_shape.ty, saved_shape.zc};
   int written = 0;
@@ -877,6 +900,7 @@ nmhd_status nmhd_slab_begin(nmhd_solver *s, double goal_time) {
 
 nmhd_status nmhd_halo_pack(nmhd_solver *s, float *send_inc, float *send_dec) {
   if (!s) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "NULL solver");
+  s->ctl_known = false;
   if (s->g.my > 0 && (!send_inc || !send_dec)) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "NULL halo buffer");
   nmhd::launch_halo_pack(s->g, s->ctl, s->w0, s->w1, send_inc, send_dec, s->stream);
   NMHD_CUDA(s, cudaGetLastError());
@@ -885,6 +909,7 @@ nmhd_status nmhd_halo_pack(nmhd_solver *s, float *send_inc, float *send_dec) {
 
 nmhd_status nmhd_halo_unpack(nmhd_solver *s, const float *recv_inc, const float *recv_dec) {
   if (!s) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "NULL solver");
+  s->ctl_known = false;
   if (s->g.my > 0 && (!recv_inc || !recv_dec)) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "NULL halo buffer");
   nmhd::launch_halo_unpack(s->g, s->ctl, s->w0, s->w1, recv_inc, recv_dec, s->stream);
   // the CFL time of this slab: every cell after a state change, else the
@@ -899,7 +924,11 @@ nmhd_status nmhd_halo_unpack(nmhd_solver *s, const float *recv_inc, const float 
   return NMHD_OK;
 }
 
-float *nmhd_cfl_slot(nmhd_solver *s) { return s ? reinterpret_cast<float *>(&s->ctl->cfl_cur) : nullptr; }
+float *nmhd_cfl_slot(nmhd_solver *s) {
+  if (!s) return nullptr;
+  s->ctl_shared = true;  // the caller may write it at any time
+  return reinterpret_cast<float *>(&s->ctl->cfl_cur);
+}
 
 nmhd_status nmhd_cfl_min(nmhd_solver *const *slabs, int n) {
   if (!slabs || n < 1 || n > nmhd::kMaxSlots) return fail(nullptr, NMHD_ERR_INVALID_ARGUMENT, "bad slab list");
@@ -917,6 +946,7 @@ nmhd_status nmhd_cfl_min(nmhd_solver *const *slabs, int n) {
 
 nmhd_status nmhd_step_stages(nmhd_solver *s) {
   if (!s) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "NULL solver");
+  s->ctl_known = false;
   if (s->cfg.time_order == 1) {
     enqueue_stage(s, 0, 1, 0, 1, s->stream);
   } else {

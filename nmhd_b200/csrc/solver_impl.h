@@ -19,6 +19,11 @@ struct nmhd_solver {
   float *w0 = nullptr, *w1 = nullptr, *wp = nullptr, *flux = nullptr, *dt_hist = nullptr;
   nmhd::StepCtl *ctl = nullptr;
   double *diag = nullptr;
+  // The control block as it stands on the device, while no enqueued work can
+  // change it (ctl_known): calls between runs then need no round trip to read
+  // it.  ctl_shared: the caller holds a pointer into it (nmhd_cfl_slot).
+  nmhd::StepCtl mirror;
+  bool ctl_known = false, ctl_shared = false;
   bool cfl_ready = false;  // ctl->cfl_cur holds the CFL time of the current state
   // 0: z-marching tiled kernels, 1: per-cell 1-D, 2: per-cell 3-D blocks,
   // 3: variant 2 as a z-chunk pipeline, 4: the variant-2 flux kernel with the
