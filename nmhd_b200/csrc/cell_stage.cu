@@ -56,6 +56,15 @@
 #define NMHD_SFLUX_MIN_BLOCKS 4
 #endif
 
+// Tiles up to which the staged flux kernel takes a CTA per tile and face axis:
+// with fewer tiles than SMs a tile's three Riemann solvers then run side by
+// side on SMs that would idle, for three times the staging.  16-step pass of a
+// 16^3 box (32 tiles) 574 -> 521 us; of boxes of 384, 576 and 768 tiles 859 ->
+// 959, 1008 -> 1190 and 1320 -> 1522 us.
+#ifndef NMHD_SPLIT_TILES
+#define NMHD_SPLIT_TILES 148
+#endif
+
 namespace nmhd {
 
 namespace {
@@ -156,23 +165,27 @@ __global__ void __launch_bounds__(kThreads, NMHD_EPI_MIN_BLOCKS)
 }
 
 // Face fluxes of one stage from a shared copy of the stage input (variant
-// 5, cell_flux_staged.cuh).
+// 5, cell_flux_staged.cuh).  kSplit: a CTA per tile and face axis (three times
+// the z blocks).
+template <bool kSplit>
 __global__ void __launch_bounds__(kThreads, NMHD_SFLUX_MIN_BLOCKS)
-    k_cell_flux_staged(const __grid_constant__ sfx::FluxMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl, const float *w0,
-                       const float *w1, const float *wp, float *__restrict__ flux, int in_sel, int half) {
+    k_cell_flux_staged(const __grid_constant__ sfx::FluxMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl,
+                       const float *w0, const float *w1, const float *wp, float *__restrict__ flux, int in_sel,
+                       int half) {
   __shared__ sfx::Smem s;
   if (ctl->done) return;
   float dt = step_dt(ctl, nullptr);
   if (half) dt = dt / 2.0f;
   const int tid = (threadIdx.z * BY + threadIdx.y) * BX + threadIdx.x;
-  const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY, z0 = blockIdx.z * BZ;
+  const int bz = kSplit ? blockIdx.z / 3 : blockIdx.z, ax = kSplit ? blockIdx.z - 3 * bz : 0;
+  const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY, z0 = bz * BZ;
   if (!sfx::stage(s, g, &maps, pick_index(ctl, in_sel), pick(ctl, in_sel, w0, w1, wp), x0, y0, z0, tid)) {
     if (tid == 0) atomicOr(&ctl->status, kStatusTimeout);
     return;
   }
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y, z = z0 + threadIdx.z;
   if (x < g.sx && y < g.sy && z < g.sz)
-    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
+    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt, ax, kSplit ? ax + 1 : 3);
 }
 
 dim3 cell_grid(const GridParams &g, int nz) {
@@ -270,8 +283,13 @@ void free_epilogue_maps(EpilogueMaps *m) { delete m; }
 void launch_cell_flux_staged(const GridParams &g, StepCtl *ctl, float *w0, float *w1, float *wp, float *flux,
                              int in_sel, int half, const EpilogueMaps *maps, cudaStream_t st) {
   static const EpilogueMaps kNone = {};  // enabled = 0: cp.async staging only
-  k_cell_flux_staged<<<cell_grid(g, g.sz), dim3(BX, BY, BZ), 0, st>>>(maps ? maps->f : kNone.f, g, ctl, w0, w1,
-                                                                      wp, flux, in_sel, half);
+  dim3 grid = cell_grid(g, g.sz);
+  const bool split = (long long)grid.x * grid.y * grid.z <= NMHD_SPLIT_TILES;
+  if (split) grid.z *= 3;
+  auto run = [&](auto kernel) {
+    kernel<<<grid, dim3(BX, BY, BZ), 0, st>>>(maps ? maps->f : kNone.f, g, ctl, w0, w1, wp, flux, in_sel, half);
+  };
+  run(split ? k_cell_flux_staged<true> : k_cell_flux_staged<false>);
 }
 
 void launch_cell_update_fused(const GridParams &g, StepCtl *ctl, float *w0, float *w1, float *wp, float *flux,
