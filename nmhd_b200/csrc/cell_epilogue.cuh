@@ -462,6 +462,41 @@ __device__ __forceinline__ void finish_cell(const Smem &s, const GridParams &g, 
   finish_cell_with<kPow2, kFinal, Ieee>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed);
 }
 
+// Columns of a tile's staged boxes that lie beyond an x edge of the box (local
+// -1 at x0 = 0, local Sx - x0 at the other edge): each is the column at the
+// other edge of the grid, one entry per row of the boxes that hold it.  Item
+// `i` of column `a` (global gx): its place in shared memory, and its value.
+struct EdgeEntry {
+  float *dst = nullptr;
+  float v;
+};
+template <class B>
+__device__ __forceinline__ bool edge_entry(EdgeEntry &e, int &i, const GridParams &g, float *dst,
+                                           const float *__restrict__ src, int nf, int a, int gx, int y0, int z0) {
+  constexpr int R = B::NJ * B::NK;
+  if (i >= R * nf) {
+    i -= R * nf;
+    return false;
+  }
+  const int f = i / R, r = i - f * R, k = r / B::NJ, j = r - k * B::NJ;
+  e.dst = dst + f * B::N + r * B::P + B::XO + (a - B::OI);
+  e.v = __ldg(src + (size_t)f * g.n + ((z0 + B::OK + k) * g.sy + (y0 + B::OJ + j)) * g.sx + gx);
+  return true;
+}
+__device__ __forceinline__ EdgeEntry edge_item(Smem &s, const GridParams &g, const float *win, const float *wb,
+                                               const float *flux, int i, bool low, int a, int gx, int y0, int z0) {
+  const size_t N = (size_t)g.n;
+  EdgeEntry e;
+  if (edge_entry<VelBox>(e, i, g, s.vel, win + N, 3, a, gx, y0, z0)) return e;
+  if (edge_entry<YXF>(e, i, g, s.bf + kYX, flux + 13 * N, 1, a, gx, y0, z0)) return e;
+  if (edge_entry<ZXF>(e, i, g, s.bf + kZX, flux + 19 * N, 1, a, gx, y0, z0)) return e;
+  if (low) return e;
+  if (edge_entry<XYF>(e, i, g, s.bf + kXY, flux + 5 * N, 1, a, gx, y0, z0)) return e;
+  if (edge_entry<XZF>(e, i, g, s.bf + kXZ, flux + 6 * N, 1, a, gx, y0, z0)) return e;
+  edge_entry<BXs>(e, i, g, s.wbf + fBX, wb + 5 * N, 1, a, gx, y0, z0);
+  return e;
+}
+
 // The whole epilogue of one tile at (x0, y0, z0); every thread of the CTA
 // calls it.  maps: the tensor maps of these buffers (interior tiles stage by
 // tensor copies), or NULL (every tile stages with cp.async).  win: stage
@@ -494,12 +529,12 @@ __device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, cons
   const unsigned vs = (unsigned)__cvta_generic_to_shared(s.vel), bs = (unsigned)__cvta_generic_to_shared(s.bf),
                  ws = (unsigned)__cvta_generic_to_shared(s.wbf),
                  mb = (unsigned)__cvta_generic_to_shared(&s.mbar);
-  // Tiles whose staged boxes (x0-4..x0+35, y0-1..y0+4, z0-1..z0+2) lie inside
-  // the box need no periodic wrap: one thread stages all of them with ten
-  // tensor copies.  The others stage entry by entry through the wrapped
-  // offset tables (16-byte row chunks when only y or z wraps).
-  const bool tma = maps && maps->enabled && x0 >= 4 && x0 + 36 <= g.sx && y0 >= 1 && y0 + 5 <= g.sy && z0 >= 1 &&
-                   z0 + 3 <= g.sz;
+  // Tiles whose staged rows and planes (y0-1..y0+4, z0-1..z0+2) lie inside the
+  // box: one thread stages all of them with ten tensor copies; at an x edge
+  // the copies leave zeros beyond it, and the one column there that is read is
+  // put in by single loads.  The others stage entry by entry through the
+  // wrapped offset tables (16-byte row chunks where rows are aligned).
+  const bool tma = maps && maps->enabled && y0 >= 1 && y0 + 5 <= g.sy && z0 >= 1 && z0 + 3 <= g.sz;
   if (tma) {
     if (tid == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
@@ -523,6 +558,10 @@ __device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, cons
     else if (tid < 40) s.gy[tid - 34] = wrap_any(y0 - 1 + (tid - 34), g.sy) * g.sx;
     else if (tid < 44) s.gz[tid - 40] = wrap_any(z0 - 1 + (tid - 40), g.sz) * g.sx * g.sy;
   }
+  const bool low = tma && x0 == 0, high = tma && x0 + BX >= g.sx;
+  EdgeEntry el, eh;
+  if (low) el = edge_item(s, g, win, wb, flux, tid, true, -1, g.sx - 1, y0, z0);
+  if (high) eh = edge_item(s, g, win, wb, flux, tid, false, g.sx - x0, 0, y0, z0);
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
   if (tma) {
@@ -540,6 +579,11 @@ __device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, cons
     }
     // every thread has passed the wait: the barrier's word is released
     if (tid == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mb) : "memory");
+    if (low || high) {
+      if (el.dst) *el.dst = el.v;
+      if (eh.dst) *eh.dst = eh.v;
+      __syncthreads();
+    }
   } else {
     // whole 16-byte row chunks where rows are 16-byte aligned
     const bool vec = (g.sx & 3) == 0;
