@@ -461,30 +461,37 @@ __device__ __forceinline__ float block_min(float v, float *red) {
   return v;
 }
 
+// The clock after a step (GlobalSetup::proceed, mhd_solver.inlrb:981): rotates
+// the state buffers and the CFL accumulators.  One thread, after every tile of
+// the final stage.
+__device__ __forceinline__ void advance_clock(StepCtl *ctl, float *dt_hist) {
+  bool last;
+  const float dts = step_dt(ctl, &last);
+  volatile StepCtl *vc = ctl;
+  const long long gen = vc->generation;
+  dt_hist[gen % kDtHistCap] = dts;
+  vc->time = vc->time + (double)dts;
+  vc->generation = gen + 1;
+  vc->parity = vc->parity ^ 1;
+  vc->cfl_cur = atomicAdd(&ctl->cfl_next, 0u);
+  vc->cfl_next = 0x7f800000u;
+  if (!(dts >= 0.0f)) atomicOr(&ctl->status, kStatusBadDt);
+  if (last || vc->status) vc->done = 1;
+  vc->blocks_done = 0;
+}
+
 // One thread folds a tile's CFL minimum and status into the box's control
-// block; the last of the box's `ntiles` tiles advances the box's clock
-// (GlobalSetup::proceed, mhd_solver.inlrb:981), rotates the state buffers and
-// the CFL accumulators.
+// block; the last of the box's `ntiles` tiles advances its clock.  ntiles 0: a
+// kernel of its own does that after the final stage.
 __device__ __forceinline__ void fold_tile(StepCtl *ctl, unsigned ntiles, float tcfl, int bad, float *dt_hist) {
   atomicMin(&ctl->cfl_next, __float_as_uint(tcfl));
   if (bad) atomicOr(&ctl->status, kStatusNumerical);
+  if (ntiles == 0) return;
   __threadfence();
   const unsigned prev = atomicAdd(&ctl->blocks_done, 1u);
   if (prev == ntiles - 1) {
     __threadfence();
-    bool last;
-    const float dts = step_dt(ctl, &last);
-    volatile StepCtl *vc = ctl;
-    const long long gen = vc->generation;
-    dt_hist[gen % kDtHistCap] = dts;
-    vc->time = vc->time + (double)dts;
-    vc->generation = gen + 1;
-    vc->parity = vc->parity ^ 1;
-    vc->cfl_cur = atomicAdd(&ctl->cfl_next, 0u);
-    vc->cfl_next = 0x7f800000u;
-    if (!(dts >= 0.0f)) atomicOr(&ctl->status, kStatusBadDt);
-    if (last || vc->status) vc->done = 1;
-    vc->blocks_done = 0;
+    advance_clock(ctl, dt_hist);
   }
 }
 

@@ -687,7 +687,7 @@ int nmhd_profile(nmhd_solver *s, int steps, double *ms_out, double *launches_out
     cnt[2] += midpoint ? flux_n : 0;
     cnt[3] += midpoint ? upd_n + ((s->cfg.flags & NMHD_FLAG_HALO_PER_STAGE) ? fills : 0) : 0;
     cnt[4] += flux_n;
-    cnt[5] += upd_n;
+    cnt[5] += upd_n + ((s->variant == 4 || s->variant == 5) && nmhd::clock_apart(g));
   }
   for (auto &e : ev) cudaEventDestroy(e);
   NMHD_CUDA(s, cudaGetLastError());

@@ -128,6 +128,9 @@ void free_epilogue_maps(EpilogueMaps *m);
 void launch_cell_update_fused(const GridParams &g, StepCtl *ctl, float *w0, float *w1, float *wp, float *flux,
                               float *dt_hist, int in_sel, int out_sel, int half, int final_stage,
                               const EpilogueMaps *maps, cudaStream_t stream);
+// Whether launch_cell_update_fused() launches a second kernel after the final
+// stage, which advances the clock.
+bool clock_apart(const GridParams &g);
 // The face fluxes of a stage from a shared-memory copy of each tile's
 // stencil (variant 5), the same fluxes as launch_cell_flux; `maps` as above
 // (interior tiles copy with one tensor copy).
