@@ -21,18 +21,17 @@ __global__ void __launch_bounds__(kThreads, 4)
     k_cell_flux_fast(const __grid_constant__ sfx::FluxMaps maps, const __grid_constant__ GridParams g, StepCtl *ctl, const float *w0,
                      const float *w1, const float *wp, float *__restrict__ flux, int in_sel, int half) {
   __shared__ sfx::Smem s;
-  if (ctl->done) return;
-  float dt = step_dt(ctl, nullptr);
-  if (half) dt = dt / 2.0f;
+  const Now now = read_now(ctl, half);
+  if (now.done) return;
   const int tid = (threadIdx.z * BY + threadIdx.y) * BX + threadIdx.x;
   const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY, z0 = blockIdx.z * BZ;
-  if (!sfx::stage(s, g, &maps, pick_index(ctl, in_sel), pick(ctl, in_sel, w0, w1, wp), x0, y0, z0, tid)) {
-    if (tid == 0) atomicOr(&ctl->status, kStatusTimeout);
+  if (!sfx::stage<true>(s, g, &maps, now.index(in_sel), now.buffer(in_sel, w0, w1, wp), x0, y0, z0, tid)) {
+    atomicOr(&ctl->status, kStatusTimeout);
     return;
   }
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y, z = z0 + threadIdx.z;
   if (x < g.sx && y < g.sy && z < g.sz)
-    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt);
+    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, now.dt);
 }
 
 }  // namespace

@@ -45,7 +45,10 @@ __device__ __forceinline__ int at(int a, int b, int c) { return ((c + 2) * NJ + 
 // lies inside the grid: one tensor copy issued by thread 0, completing on the
 // mbarrier (bounded wait; false if it timed out).  Others: cp.async through
 // the wrapped offset tables, 16-byte row chunks where Sx % 4 == 0, else entry
-// by entry.  Every thread of the CTA calls it.
+// by entry.  Every thread of the CTA calls it.  kOnce: the CTA stages no other
+// tile, so a thread goes on when it has seen the copy land (and the answer is
+// the thread's own).
+template <bool kOnce = false>
 __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMaps *maps, int buf,
                                       const float *__restrict__ w, int x0, int y0, int z0, int tid) {
   const size_t N = (size_t)g.n;
@@ -66,6 +69,9 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
           : "memory");
     }
     __syncthreads();
+    // (a second bounded wait where the first gives up: no copy may still be
+    // writing when the CTA exits)
+    if (kOnce) return epi::mbar_wait_bounded(mb) || (epi::mbar_wait_bounded(mb), false);
     const bool ok = __syncthreads_and(epi::mbar_wait_bounded(mb));
     if (!ok) {
       // flag it and wait once more (bounded) so that no copy is still

@@ -72,6 +72,37 @@ __device__ __forceinline__ float step_dt(const StepCtl *c, bool *last) {
   return dt;
 }
 
+// What a stage kernel needs of the control block.  All of it is loaded before
+// any of it is tested, so that a CTA waits for one round trip to L2 and not for
+// one after another; `half` halves the time step.
+struct Now {
+  int done, parity;
+  float dt;
+  // Buffer index (0 w0, 1 w1, 2 predictor) of selector `sel` (0 current, 1
+  // next, 2 predictor), and the buffer.
+  __device__ __forceinline__ int index(int sel) const { return sel == 2 ? 2 : (sel == 0) == (parity == 0) ? 0 : 1; }
+  template <class T>
+  __device__ __forceinline__ T *buffer(int sel, T *w0, T *w1, T *wp) const {
+    const int i = index(sel);
+    return i == 2 ? wp : i == 0 ? w0 : w1;
+  }
+};
+__device__ __forceinline__ Now read_now(const StepCtl *ctl, int half) {
+  StepCtl c;
+  c.time = ctl->time;
+  c.generation = ctl->generation;
+  c.cfl_cur = ctl->cfl_cur;
+  c.goal = ctl->goal;
+  c.dt_seq = ctl->dt_seq;
+  c.dt_seq_base = ctl->dt_seq_base;
+  Now now = {ctl->done, ctl->parity, 0.0f};
+  asm volatile("" : "+r"(now.done), "+r"(now.parity), "+d"(c.time), "+l"(c.generation), "+r"(c.cfl_cur), "+f"(c.goal),
+               "+l"(c.dt_seq), "+l"(c.dt_seq_base));
+  now.dt = now.done ? 0.0f : step_dt(&c, nullptr);
+  if (half) now.dt = now.dt / 2.0f;
+  return now;
+}
+
 // Loads of face_flux's inputs: read-only global memory (the stage input in
 // HBM) or a plain load (a shared-memory copy of it).
 struct GlobalLd {

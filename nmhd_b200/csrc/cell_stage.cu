@@ -154,19 +154,18 @@ __global__ void __launch_bounds__(kThreads, NMHD_EPI_MIN_BLOCKS)
                     float *w0, float *w1, float *wp, const float *__restrict__ flux, float *dt_hist, int in_sel,
                     int out_sel, int half, unsigned ntiles) {
   __shared__ epi::Smem s;
-  if (ctl->done) return;
-  float dt = step_dt(ctl, nullptr);
-  if (half) dt = dt / 2.0f;
-  const float *win = pick(ctl, in_sel, w0, w1, wp), *wb = pick(ctl, 0, w0, w1, wp);
-  float *wo = const_cast<float *>(pick(ctl, out_sel, w0, w1, wp));
+  const Now now = read_now(ctl, half);
+  if (now.done) return;
+  const float *win = now.buffer(in_sel, w0, w1, wp), *wb = now.buffer(0, w0, w1, wp);
+  float *wo = now.buffer(out_sel, w0, w1, wp);
   int bad = 0, timed_out = 0;
   // tiles in the reverse of the flux kernel's order: CTAs are dispatched in
   // block order, so the first tiles read the fluxes written last, which are
   // still in L2
   const int tx = gridDim.x - 1 - blockIdx.x, ty = gridDim.y - 1 - blockIdx.y, tz = gridDim.z - 1 - blockIdx.z;
   float speed[3] = {0.0f, 0.0f, 0.0f};
-  epi::tile_epilogue<kPow2, kFinal>(s, g, &maps, pick_index(ctl, in_sel), pick_index(ctl, 0), win, wb, wo, flux,
-                                    tx * BX, ty * BY, tz * BZ, dt, &bad, &timed_out, speed);
+  epi::tile_epilogue<kPow2, kFinal>(s, g, &maps, now.index(in_sel), now.index(0), win, wb, wo, flux, tx * BX,
+                                    ty * BY, tz * BZ, now.dt, &bad, &timed_out, speed);
   if (timed_out && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0)
     atomicOr(&ctl->status, kStatusTimeout);
   if (kFinal) finish_tile_speeds(g, ctl, ntiles, speed, bad, dt_hist, s.red);
@@ -185,19 +184,18 @@ __global__ void __launch_bounds__(kThreads, NMHD_SFLUX_MIN_BLOCKS)
                        const float *w0, const float *w1, const float *wp, float *__restrict__ flux, int in_sel,
                        int half) {
   __shared__ sfx::Smem s;
-  if (ctl->done) return;
-  float dt = step_dt(ctl, nullptr);
-  if (half) dt = dt / 2.0f;
+  const Now now = read_now(ctl, half);
+  if (now.done) return;
   const int tid = (threadIdx.z * BY + threadIdx.y) * BX + threadIdx.x;
   const int bz = kSplit ? blockIdx.z / 3 : blockIdx.z, ax = kSplit ? blockIdx.z - 3 * bz : 0;
   const int x0 = blockIdx.x * BX, y0 = blockIdx.y * BY, z0 = bz * BZ;
-  if (!sfx::stage(s, g, &maps, pick_index(ctl, in_sel), pick(ctl, in_sel, w0, w1, wp), x0, y0, z0, tid)) {
-    if (tid == 0) atomicOr(&ctl->status, kStatusTimeout);
+  if (!sfx::stage<true>(s, g, &maps, now.index(in_sel), now.buffer(in_sel, w0, w1, wp), x0, y0, z0, tid)) {
+    atomicOr(&ctl->status, kStatusTimeout);
     return;
   }
   const int x = x0 + threadIdx.x, y = y0 + threadIdx.y, z = z0 + threadIdx.z;
   if (x < g.sx && y < g.sy && z < g.sz)
-    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, dt, ax, kSplit ? ax + 1 : 3);
+    sfx::flux_cell_staged(g, s.w, flux, threadIdx.x, threadIdx.y, threadIdx.z, x, y, z, now.dt, ax, kSplit ? ax + 1 : 3);
 }
 
 dim3 cell_grid(const GridParams &g, int nz) {
