@@ -290,10 +290,11 @@ int nmhd_batch_launches_per_step(const nmhd_batch *b);
  * compiled for that shape (fewer registers), 0 runs every box in one launch of
  * the general form (half the launches: better for many small boxes).
  * kernel = 3 is the fused pass: split = 1 runs constrained transport and the
- * conserved update of the 32 x 4 x 2 boxes as one kernel (the single-box fused
+ * conserved update as one kernel for the boxes that 32 x 4 x 2 tiles cover with
+ * at most a third more padded cells than their own tile (the single-box fused
  * epilogue; it takes effect while kernels 1 and 2 are split), persistent its
  * schedule; split = 0 (the default) turns it off.  kernel = 4 is the staged
- * flux pass: split = 1 computes the face fluxes of the 32 x 4 x 2 boxes from a
+ * flux pass: split = 1 computes the face fluxes of the same boxes from a
  * shared-memory copy of each tile's stencil (the single-box variant-5 flux
  * kernel; it takes effect while kernel 0 is split), persistent its schedule. */
 nmhd_status nmhd_batch_set_schedule(nmhd_batch *b, int kernel, int persistent, int split);
@@ -307,7 +308,8 @@ nmhd_status nmhd_batch_set_schedule(nmhd_batch *b, int kernel, int persistent, i
  * unchanged.  trials_out (may be NULL) receives up to max_trials rows of
  * (kernel, persistent, split, ms per launch), the two comparisons as rows
  * (4, persistent, staged, ms per flux launch) and (3, persistent, fused, ms
- * per stage update).  Returns the number of rows written or a negative
+ * per stage update; with the passes on, only where a box's own tile is 32 x 4 x
+ * 2).  Returns the number of rows written or a negative
  * nmhd_status.
  * Every schedule gives bitwise the same result. */
 int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_trials);

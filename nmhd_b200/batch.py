@@ -141,9 +141,10 @@ class BatchSolver:
         transport, 2 conserved update): persistent or one tile per CTA; with
         ``split`` the boxes with 32 x 4 x 2 tiles run in a launch of their own.
         ``kernel`` 3 is the fused pass (constrained transport and conserved
-        update of the 32 x 4 x 2 boxes in one kernel): ``split`` turns it on
+        update in one kernel, for the boxes that 32 x 4 x 2 tiles cover with at
+        most a third more padded cells than their own): ``split`` turns it on
         (it then needs kernels 1 and 2 split), ``persistent`` its schedule.
-        ``kernel`` 4 is the staged flux pass of the 32 x 4 x 2 boxes (their
+        ``kernel`` 4 is the staged flux pass of the same boxes (their
         fluxes from a shared copy of each tile's stencil; needs kernel 0
         split), turned on and scheduled the same way."""
         self._check(self._L.nmhd_batch_set_schedule(self._h, int(kernel), int(bool(persistent)),
