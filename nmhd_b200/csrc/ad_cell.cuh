@@ -582,7 +582,12 @@ NMHD_HD void a_flux_face(const GGrid<R> &g, const R *win, const R *lamBn, const 
   face_input_nb<AX>(g, win, nb, y, h, in, bn, &ch);
   HState<R> ls;
   R lbn;
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(R) == sizeof(float)) hlld_adjoint_ranged(g.gamma, bn, in, lf, ls, lbn);
+  else hlld_adjoint(g.gamma, bn, in, lf, ls, lbn);
+#else
   hlld_adjoint(g.gamma, bn, in, lf, ls, lbn);
+#endif
   // Transpose of the reconstruction of each variable at this face, split by
   // the four cells x0..x3 (= face - 2 .. face + 1 along AX) it reads:
   // left = x1 + d1/2 with d1 = 0 | x1 - x0 | x2 - x1, right = x2 - d2/2 with

@@ -14,9 +14,34 @@
 // step below; every forward intermediate is read from the tape.
 #pragma once
 #include "ad_scalar.cuh"
+#include "rounded.cuh"
 
 namespace nmhd {
 namespace ad {
+
+// Arithmetic of the quotients and roots.  OfType: the scalar type's own.
+// OfRanges (float): one reciprocal per denominator and no range test of each
+// quotient (rounded.cuh); where hold() says that every operand was in range, the
+// tape and the adjoint are bit for bit OfType's, else they are taken again with
+// it.
+template <class T>
+struct OfType {
+  static constexpr bool kRanged = false;
+  typedef T Den;
+  NMHD_HD static void positive(const T &) {}
+  NMHD_HD static Den under(const T &b) { return b; }
+  NMHD_HD static T ratio(const T &a, const Den &d) { return a / d; }
+  NMHD_HD static T div(const T &a, const Den &d) { return a / d; }
+  NMHD_HD static T div_bounded(const T &a, const Den &d) { return a / d; }
+  NMHD_HD static T root(const T &x) { return gsqrt(x); }
+  NMHD_HD static T inv(const T &x) { return T(1) / x; }
+  NMHD_HD static bool hold() { return true; }
+};
+struct OfRanges : Ranged {
+  static constexpr bool kRanged = true;
+  typedef Denominator Den;
+  NMHD_HD static float inv(float x) { return inverse(x); }
+};
 
 // Left/right Riemann states: rho, v_n, v_t1, v_t2, p, B_t1, B_t2.
 template <class T>
@@ -40,49 +65,61 @@ struct HTape {
   int region;
 };
 
-template <class T>
-NMHD_HD void hlld_side_pre(const T gamma, const T gm1, const T Bx, const T B2x, HSide<T> &s) {
+template <class T, class A>
+NMHD_HD void hlld_side_pre(A &q, const T gamma, const typename A::Den &gm1, const T B2x, HSide<T> &s) {
   typedef typename Traits<T>::wide W;
   s.mx = s.d * s.u;
   s.my = s.d * s.v;
   s.mz = s.d * s.w;
   s.B2 = B2x + s.by * s.by + s.bz * s.bz;
   s.v2 = s.u * s.u + s.v * s.v + s.w * s.w;
-  // etot = p/(gamma-1) + 0.5*rho*v2 + 0.5*B2, the last two terms in double
-  s.e = to<T>(to<W>(s.p / gm1) + W(0.5) * to<W>(s.d) * to<W>(s.v2) + W(0.5) * to<W>(s.B2));
+  q.positive(s.d);
+  q.positive(s.p);
+  const T heat = q.ratio(s.p, gm1);
   s.gp = gamma * s.p;
   s.gpb = s.gp + s.B2;
+  q.positive(s.gpb);
   s.disc = s.gpb * s.gpb - T(4.0f) * s.gp * B2x;
-  s.sq = gsqrt(s.disc);
+  s.sq = q.root(s.disc);
   s.num = s.gpb + s.sq;
-  s.cf = gsqrt(s.num / (T(2.0f) * s.d));
-  s.pT = to<T>(to<W>(s.p) + W(0.5) * to<W>(s.B2));
-  (void)Bx;
+  s.cf = q.root(q.ratio(s.num, q.under(T(2.0f) * s.d)));
+  // etot = p/(gamma-1) + 0.5*rho*v2 + 0.5*B2, the last two terms in double
+  // (each exact, so that a fused multiply-add rounds as the addition does)
+  if constexpr (A::kRanged) {
+    s.e = (float)fma(0.5, (double)s.B2, fma(0.5, (double)s.d * (double)s.v2, (double)heat));
+    s.pT = fmaf(0.5f, s.B2, s.p);
+  } else {
+    s.e = to<T>(to<W>(heat) + W(0.5) * to<W>(s.d) * to<W>(s.v2) + W(0.5) * to<W>(s.B2));
+    s.pT = to<T>(to<W>(s.p) + W(0.5) * to<W>(s.B2));
+  }
 }
 
-// Star state of one side; S = S_L or S_R, sign = -1 (left) or +1 (right).
-template <class T>
-NMHD_HD void hlld_side_star(const T Bx, const T B2x, const T TINY, const T S, const T S_M, HSide<T> &s) {
+// Star state of one side; S = S_L or S_R.
+template <class T, class A>
+NMHD_HD void hlld_side_star(A &q, const T Bx, const T B2x, const T TINY, const T S, const T S_M, const T pT_s,
+                            HSide<T> &s) {
   s.sm = S - S_M;
-  s.ds = s.d * s.sv / s.sm;
-  s.dn = s.d * s.sv * s.sm - B2x + TINY;
-  s.vs = s.v - Bx * s.by * (S_M - s.u) / s.dn;
-  s.ws = s.w - Bx * s.bz * (S_M - s.u) / s.dn;
+  q.positive(gabs(s.sm));
+  const typename A::Den sm = q.under(s.sm);
+  const T dsv = s.d * s.sv;
+  s.ds = q.ratio(dsv, sm);
+  q.positive(s.ds);
+  s.dn = dsv * s.sm - B2x + TINY;
+  q.positive(s.dn);
+  const typename A::Den dn = q.under(s.dn);
+  s.vs = s.v - q.div(Bx * s.by * (S_M - s.u), dn);
+  s.ws = s.w - q.div(Bx * s.bz * (S_M - s.u), dn);
   s.q = s.d * (s.sv * s.sv) - B2x;
-  s.bys = s.by * s.q / s.dn;
-  s.bzs = s.bz * s.q / s.dn;
-}
-
-template <class T>
-NMHD_HD void hlld_side_energy(const T Bx, const T S_M, const T pT_s, HSide<T> &s) {
+  s.bys = q.div(s.by * s.q, dn);
+  s.bzs = q.div(s.bz * s.q, dn);
   s.vB = s.u * Bx + s.v * s.by + s.w * s.bz;
   s.vBs = S_M * Bx + s.vs * s.bys + s.ws * s.bzs;
-  s.es = (s.sv * s.e - s.pT * s.u + pT_s * S_M + Bx * (s.vB - s.vBs)) / s.sm;
-  s.sd = gsqrt(s.ds);
+  s.es = q.div_bounded(s.sv * s.e - s.pT * s.u + pT_s * S_M + Bx * (s.vB - s.vBs), sm);
+  s.sd = q.root(s.ds);
 }
 
-template <class T>
-NMHD_HD void hlld_tape(const T gamma, const T Bx, const HState<T> &in, HTape<T> &t) {
+template <class T, class A>
+NMHD_HD void hlld_tape(A &q, const T gamma, const T Bx, const HState<T> &in, HTape<T> &t) {
   typedef typename Traits<T>::wide W;
   typedef typename Traits<T>::real R;
   const T TINY = to<T>((R)1.0e-10);
@@ -93,28 +130,38 @@ NMHD_HD void hlld_tape(const T gamma, const T Bx, const HState<T> &in, HTape<T> 
   t.L.d = in.dl; t.L.u = in.ul; t.L.v = in.vl; t.L.w = in.wl; t.L.p = in.pl; t.L.by = in.byl; t.L.bz = in.bzl;
   t.R.d = in.dr; t.R.u = in.ur; t.R.v = in.vr; t.R.w = in.wr; t.R.p = in.pr; t.R.by = in.byr; t.R.bz = in.bzr;
   t.B2x = Bx * Bx;
-  const T gm1 = gamma - T(1.0f);
-  hlld_side_pre(gamma, gm1, Bx, t.B2x, t.L);
-  hlld_side_pre(gamma, gm1, Bx, t.B2x, t.R);
+  const typename A::Den gm1 = q.under(gamma - T(1.0f));
+  hlld_side_pre(q, gamma, gm1, t.B2x, t.L);
+  hlld_side_pre(q, gamma, gm1, t.B2x, t.R);
+  if constexpr (A::kRanged) q.positive(fminf(t.L.disc, t.R.disc) >= 0x1p-90f ? 1.0f : 0.0f);
   const T fsig = to<T>(1.41421354f);  // (float)sqrt(2.0) in both reference builds
   t.cfmax = fsig * gmax(t.L.cf, t.R.cf);
   t.S_L = gmin(t.L.u, t.R.u) - t.cfmax;
   t.S_R = gmax(t.L.u, t.R.u) + t.cfmax;
   t.R.sv = t.S_R - t.R.u;
   t.L.sv = t.S_L - t.L.u;
+  q.positive(t.R.sv);
+  q.positive(-t.L.sv);
   t.den = t.R.sv * t.R.d - t.L.sv * t.L.d;
-  const W rden = W(1.0) / to<W>(t.den);
+  q.positive(t.den);
   t.SMn = t.R.sv * t.R.mx - t.L.sv * t.L.mx - t.R.pT + t.L.pT;
-  t.S_M = to<T>(to<W>(t.SMn) * rden);
   t.pTn = t.R.sv * t.R.d * t.L.pT - t.L.sv * t.L.d * t.R.pT;
   t.pTn = t.pTn + t.L.d * t.R.d * t.R.sv * t.L.sv * (t.R.u - t.L.u);
-  t.pT_s = to<T>(to<W>(t.pTn) * rden);
-  hlld_side_star(Bx, t.B2x, TINY, t.S_L, t.S_M, t.L);
-  hlld_side_star(Bx, t.B2x, TINY, t.S_R, t.S_M, t.R);
-  hlld_side_energy(Bx, t.S_M, t.pT_s, t.L);
-  hlld_side_energy(Bx, t.S_M, t.pT_s, t.R);
-  t.L.Ss = t.S_M - t.absBx / t.L.sd;
-  t.R.Ss = t.S_M + t.absBx / t.R.sd;
+  if constexpr (A::kRanged) {
+    // the product with a double reciprocal rounds to the float quotient
+    // (hlld_flux_with(), mhd_math.cuh)
+    const Denominator den = q.under(t.den);
+    t.S_M = q.div_bounded(t.SMn, den);
+    t.pT_s = q.div_bounded(t.pTn, den);
+  } else {
+    const W rden = W(1.0) / to<W>(t.den);
+    t.S_M = to<T>(to<W>(t.SMn) * rden);
+    t.pT_s = to<T>(to<W>(t.pTn) * rden);
+  }
+  hlld_side_star(q, Bx, t.B2x, TINY, t.S_L, t.S_M, t.pT_s, t.L);
+  hlld_side_star(q, Bx, t.B2x, TINY, t.S_R, t.S_M, t.pT_s, t.R);
+  t.L.Ss = t.S_M - q.div(t.absBx, q.under(t.L.sd));
+  t.R.Ss = t.S_M + q.div(t.absBx, q.under(t.R.sd));
   const R SL = val(t.S_L), SLs = val(t.L.Ss), SM = val(t.S_M), SRs = val(t.R.Ss), SR = val(t.S_R);
   int region;
   if (SL > R(0)) region = 0;
@@ -126,16 +173,22 @@ NMHD_HD void hlld_tape(const T gamma, const T Bx, const HState<T> &in, HTape<T> 
   t.region = region;
   if (region == 2 || region == 3) {
     const T sgn = t.sgn;
-    t.fr = T(1.0f) / (t.L.sd + t.R.sd);
+    t.fr = q.inv(t.L.sd + t.R.sd);
     t.vss = t.fr * (t.L.sd * t.L.vs + t.R.sd * t.R.vs + (t.R.bys - t.L.bys) * sgn);
     t.wss = t.fr * (t.L.sd * t.L.ws + t.R.sd * t.R.ws + (t.R.bzs - t.L.bzs) * sgn);
-    t.sdLR = gsqrt(t.L.ds * t.R.ds);
+    t.sdLR = q.root(t.L.ds * t.R.ds);
     t.Byss = t.fr * (t.L.sd * t.R.bys + t.R.sd * t.L.bys + t.sdLR * (t.R.vs - t.L.vs) * sgn);
     t.Bzss = t.fr * (t.L.sd * t.R.bzs + t.R.sd * t.L.bzs + t.sdLR * (t.R.ws - t.L.ws) * sgn);
     t.vBss = t.S_M * Bx + t.vss * t.Byss + t.wss * t.Bzss;
     t.eLss = t.L.es - t.L.sd * (t.L.vBs - t.vBss) * sgn;
     t.eRss = t.R.es + t.R.sd * (t.R.vBs - t.vBss) * sgn;
   }
+}
+
+template <class T>
+NMHD_HD void hlld_tape(const T gamma, const T Bx, const HState<T> &in, HTape<T> &t) {
+  OfType<T> q;
+  hlld_tape(q, gamma, Bx, in, t);
 }
 
 // The flux of the region on the tape (hlld.inl:229-284); kLeft selects the
@@ -209,12 +262,12 @@ NMHD_HD void hadj_zero(HAdj<R> &a) {
 // Reverse of hlld_side_energy and hlld_side_star for one side.  The reverse
 // sweep needs no correctly rounded quotients: each denominator is inverted
 // once and multiplied (the forward tape above keeps the exact divisions).
-template <class R>
+template <class A, class R>
 NMHD_HD void hlld_side_star_rev(const HSide<R> &s, const R Bx, const R S_M, const R pT_s, HAdj<R> &a, R &aSM,
                                 R &apTs, R &aBx, R &aB2x, R &aS) {
-  const R ism = R(1) / s.sm, idn = R(1) / s.dn;
+  const R ism = A::inv(s.sm), idn = A::inv(s.dn);
   // sd = sqrt(ds)
-  if (s.sd > R(0)) a.ds += a.sd * (R(0.5) / s.sd);
+  if (s.sd > R(0)) a.ds += a.sd * (R(0.5) * A::inv(s.sd));
   // es = (sv*e - pT*u + pT_s*S_M + Bx*(vB - vBs)) / sm
   {
     const R t = a.es * ism;
@@ -288,7 +341,7 @@ NMHD_HD void hlld_side_vB_rev(const HSide<R> &s, const R Bx, HAdj<R> &a, R &aBx)
 }
 
 // Reverse of hlld_side_pre (after pT, cf, e, mx.. have their adjoints).
-template <class R>
+template <class A, class R>
 NMHD_HD void hlld_side_pre_rev(const HSide<R> &s, const R gamma, const R igm1, const R B2x, HAdj<R> &a,
                                R &aB2x) {
   // pT = p + 0.5*B2
@@ -296,15 +349,15 @@ NMHD_HD void hlld_side_pre_rev(const HSide<R> &s, const R gamma, const R igm1, c
   a.B2 = fmaa(R(0.5), a.pT, a.B2);
   // cf = sqrt(num/(2d))
   if (s.cf > R(0)) {
-    const R id = R(1) / s.d;
-    const R aQ = a.cf * (R(0.5) / s.cf);
+    const R id = A::inv(s.d);
+    const R aQ = a.cf * (R(0.5) * A::inv(s.cf));
     const R Q = R(0.5) * s.num * id;
     const R anum = R(0.5) * aQ * id;
     a.d = fmaa(-(aQ * Q), id, a.d);
     // num = gpb + sq; sq = sqrt(disc); disc = gpb^2 - 4 gp B2x; gpb = gp + B2
     R agpb = anum, agp = R(0);
     if (s.sq > R(0)) {
-      const R adisc = anum * (R(0.5) / s.sq);
+      const R adisc = anum * (R(0.5) * A::inv(s.sq));
       agpb = fmaa(adisc * R(2), s.gpb, agpb);
       agp = fmaa(-(adisc * R(4)), B2x, agp);
       aB2x = fmaa(-(adisc * R(4)), s.gp, aB2x);
@@ -339,7 +392,7 @@ NMHD_HD void hlld_side_pre_rev(const HSide<R> &s, const R gamma, const R igm1, c
 // carries the two sides' mirror formulas (S_L* = S_M - |Bx|/sdL vs S_R* = S_M
 // + |Bx|/sdR, eL** = eL* - sdL(...) vs eR** = eR* + sdR(...)).  Faces of one
 // warp with fan regions on both sides then take one path.
-template <class R>
+template <class A, class R>
 NMHD_HD void hlld_region_rev(const HTape<R> &t, const R lf[7], HAdj<R> &aL, HAdj<R> &aR, R &aBx, R &aB2x,
                              R &aSM, R &aSL, R &aSR, R &aabs) {
   const int rg = t.region;
@@ -464,7 +517,7 @@ NMHD_HD void hlld_region_rev(const HTape<R> &t, const R lf[7], HAdj<R> &aL, HAdj
       }
       // sdLR = sqrt(dLs*dRs)
       if (t.sdLR > R(0)) {
-        const R c = asdLR * (R(0.5) / t.sdLR);
+        const R c = asdLR * (R(0.5) * A::inv(t.sdLR));
         aL.ds = fmaa(c, t.R.ds, aL.ds);
         aR.ds = fmaa(c, t.L.ds, aR.ds);
       }
@@ -477,7 +530,7 @@ NMHD_HD void hlld_region_rev(const HTape<R> &t, const R lf[7], HAdj<R> &aL, HAdj
       // Sss = S_M + sx*|Bx|/sdX
       aSM += aSss;
       {
-        const R isd = R(1) / sd;
+        const R isd = A::inv(sd);
         aabs = fmaa(sx * aSss, isd, aabs);
         aX.sd = fmaa(-(sx * aSss * t.absBx * isd), isd, aX.sd);
       }
@@ -502,27 +555,29 @@ NMHD_HD void hlld_region_rev(const HTape<R> &t, const R lf[7], HAdj<R> &aL, HAdj
   aSR = fmaa(kr, aSX, aSR);
 }
 
-// Adjoint of hlld_g: ls and lBx receive d<lf, f>/d(state) and d<lf, f>/dBx.
-template <class R>
-NMHD_HD void hlld_adjoint(const R gamma, const R Bx, const HState<R> &in, const R lf[7], HState<R> &ls,
-                          R &lBx) {
+// Adjoint of hlld_g in the arithmetic A: ls and lBx receive d<lf, f>/d(state)
+// and d<lf, f>/dBx; false where A does not cover an operand.
+template <class A, class R>
+NMHD_HD bool hlld_adjoint_with(const R gamma, const R Bx, const HState<R> &in, const R lf[7], HState<R> &ls,
+                               R &lBx) {
   HTape<R> t;
-  hlld_tape(gamma, Bx, in, t);
+  A q;
+  hlld_tape(q, gamma, Bx, in, t);
   const int rg = t.region;
   HAdj<R> aL, aR;
   hadj_zero(aL);
   hadj_zero(aR);
   R aBx = R(0), aB2x = R(0), aSM = R(0), apTs = R(0), aSL = R(0), aSR = R(0), aabs = R(0);
   const R sgn = t.sgn;
-  hlld_region_rev(t, lf, aL, aR, aBx, aB2x, aSM, aSL, aSR, aabs);
+  hlld_region_rev<A>(t, lf, aL, aR, aBx, aB2x, aSM, aSL, aSR, aabs);
   if (rg != 0 && rg != 5) {  // regions 0 and 5 use no wave speed or star state
     // --- star states of both sides ---------------------------------------------
-    hlld_side_star_rev(t.L, Bx, t.S_M, t.pT_s, aL, aSM, apTs, aBx, aB2x, aSL);
-    hlld_side_star_rev(t.R, Bx, t.S_M, t.pT_s, aR, aSM, apTs, aBx, aB2x, aSR);
+    hlld_side_star_rev<A>(t.L, Bx, t.S_M, t.pT_s, aL, aSM, apTs, aBx, aB2x, aSL);
+    hlld_side_star_rev<A>(t.R, Bx, t.S_M, t.pT_s, aR, aSM, apTs, aBx, aB2x, aSR);
 
     // --- S_M = SMn/den, pT* = pTn/den ---------------------------------------------
     {
-      const R iden = R(1) / t.den;
+      const R iden = A::inv(t.den);
       const R aSMn = aSM * iden, apTn = apTs * iden;
       const R aden = -(aSM * t.S_M + apTs * t.pT_s) * iden;
       const R dl = t.L.d, dr = t.R.d, sLv = t.L.sv, sRv = t.R.sv, du = t.R.u - t.L.u;
@@ -563,16 +618,45 @@ NMHD_HD void hlld_adjoint(const R gamma, const R Bx, const HState<R> &in, const 
   }
   hlld_side_vB_rev(t.L, Bx, aL, aBx);
   hlld_side_vB_rev(t.R, Bx, aR, aBx);
-  const R igm1 = R(1) / (gamma - R(1));
-  hlld_side_pre_rev(t.L, gamma, igm1, t.B2x, aL, aB2x);
-  hlld_side_pre_rev(t.R, gamma, igm1, t.B2x, aR, aB2x);
+  const R igm1 = A::inv(gamma - R(1));
+  hlld_side_pre_rev<A>(t.L, gamma, igm1, t.B2x, aL, aB2x);
+  hlld_side_pre_rev<A>(t.R, gamma, igm1, t.B2x, aR, aB2x);
   aBx = fmaa(aabs, sgn, fmaa(R(2) * Bx, aB2x, aBx));
 
   ls.dl = aL.d; ls.dr = aR.d; ls.ul = aL.u; ls.ur = aR.u; ls.vl = aL.v; ls.vr = aR.v;
   ls.wl = aL.w; ls.wr = aR.w; ls.pl = aL.p; ls.pr = aR.p; ls.byl = aL.by; ls.byr = aR.by;
   ls.bzl = aL.bz; ls.bzr = aR.bz;
   lBx = aBx;
+  return q.hold();
 }
+
+template <class R>
+NMHD_HD void hlld_adjoint(const R gamma, const R Bx, const HState<R> &in, const R lf[7], HState<R> &ls, R &lBx) {
+  hlld_adjoint_with<OfType<R>>(gamma, Bx, in, lf, ls, lBx);
+}
+
+#ifdef __CUDACC__
+// FP32 on the GPU.  The second taking is a call, so that its registers and code
+// stay out of the passes that seldom need it.
+struct HAdjoint {
+  HState<float> s;
+  float bx;
+};
+static __device__ __noinline__ HAdjoint hlld_adjoint_of_type(float gamma, float Bx, HState<float> in, float l0, float l1,
+                                                             float l2, float l3, float l4, float l5, float l6) {
+  const float lf[7] = {l0, l1, l2, l3, l4, l5, l6};
+  HAdjoint o;
+  hlld_adjoint_with<OfType<float>>(gamma, Bx, in, lf, o.s, o.bx);
+  return o;
+}
+static __device__ __forceinline__ void hlld_adjoint_ranged(const float gamma, const float Bx, const HState<float> &in,
+                                                           const float lf[7], HState<float> &ls, float &lBx) {
+  if (hlld_adjoint_with<OfRanges>(gamma, Bx, in, lf, ls, lBx) && denominator_in_range(gamma - 1.0f)) return;
+  const HAdjoint o = hlld_adjoint_of_type(gamma, Bx, in, lf[0], lf[1], lf[2], lf[3], lf[4], lf[5], lf[6]);
+  ls = o.s;
+  lBx = o.bx;
+}
+#endif
 
 }  // namespace ad
 }  // namespace nmhd
