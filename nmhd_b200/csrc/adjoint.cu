@@ -10,7 +10,7 @@
 //
 // Memory: checkpoints (8 fields) every K steps, plus the tape (24 fields per
 // step: filled input, predictor, raw output) of the last segments, one shared
-// 21-field flux scratch, plus 3 adjoint states and 42 scratch fields.  The forward run
+// 21-field flux scratch, plus 3 adjoint states and 28 scratch fields.  The forward run
 // keeps as many trailing segments on the tape as the tape budget allows (at
 // least one; by default as many as fit in half of the free device memory),
 // and the reverse sweep recomputes only the earlier segments, from their
