@@ -108,22 +108,18 @@ struct EpiMaps {
   int enabled;
 };
 
-// Global offset of tile-local cell (a, b, c) through the wrapped tables.
-__device__ __forceinline__ int goff(const Smem &s, int a, int b, int c) {
-  return s.gz[c + 1] + s.gy[b + 1] + s.gx[a + 1];
-}
-
-// One 4-byte asynchronous global-to-shared copy (cp.async, sm_80 and later):
-// no register holds the value while it is in flight.
-__device__ __forceinline__ void cp_async4(unsigned dst, const float *src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+// One asynchronous global-to-shared copy of W floats (cp.async, sm_80 and
+// later; both addresses aligned to them): no register holds the value while it
+// is in flight.  16 bytes are cached in L2 only.
+template <int W>
+__device__ __forceinline__ void cp_async(unsigned dst, const float *src) {
+  static_assert(W == 1 || W == 2 || W == 4, "4, 8 or 16 bytes");
+  if constexpr (W == 4)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(4 * W) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// 16-byte asynchronous copy (both addresses 16-byte aligned), cached in L2 only.
-__device__ __forceinline__ void cp_async16(unsigned dst, const float *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
 
 // Tensor copy of box B at tile origin (x0, y0, z0), fields f0.., into shared
 // address dst, completing on the tile's mbarrier (cp.async.bulk.tensor; the
@@ -161,48 +157,69 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned mbar) {
 
 // Copy box B of global field src (and, for F > 1 fields, the fields at
 // strides of N after it) into shared memory at dst (a shared-space address;
-// field f at dst + 4 * f * B::N) with asynchronous copies, so every copy of
-// the tile is issued before the first is waited for.
-//  vec (rows 16-byte aligned, Sx % 4 == 0): whole padded rows, x0 + OI - XO
-//  .. + P - 1, 16 bytes per copy, the tile's threads over all (row, 16-byte
-//  chunk) pairs; a chunk that lies beyond an x edge of the box is the chunk
-//  Sx away (the periodic wrap moves whole, still aligned, 4-float chunks);
-//  otherwise: entry by entry, one row per warp at a time (the row's y and z
-//  offsets warp-uniform, a lane's x offsets from the wrapped table).
-template <class B, int F>
+// field f at dst + 4 * f * B::N) with asynchronous copies of W floats (Sx % W
+// == 0), so every copy of the tile is issued before the first is waited for.
+//  W > 1: the tile's threads over all (row, chunk) pairs of the entries; a
+//  chunk that lies beyond an x edge of the box is the (still aligned) chunk Sx
+//  away;
+//  W = 1: one row per warp at a time (the row's y and z offsets warp-uniform, a
+//  lane's x offsets from the wrapped table).
+// Both kernels' staging issues what it copies: with 8-byte copies where only
+// pairs are aligned a 250x97x61 box took 142 us a flux launch (4-byte copies:
+// 169) and 116 / 134 us an update (128 / 146).  With W = 1 over all entries the
+// update of a 251x97x61 box took 138 / 157 us instead of 128 / 148.
+template <class B, int F, int W>
 __device__ __forceinline__ void load_box(const Smem &s, unsigned dst, const float *__restrict__ src, size_t N,
-                                         int x0, int nx, bool vec, int tid) {
-  if (vec) {
-    constexpr int PV = B::P / 4, R = B::NJ * B::NK;
-    const int xs = x0 + B::OI - B::XO;
-    for (int e = tid; e < R * PV; e += kThreads) {
-      const int r = e / PV, v = e - r * PV;
+                                         int x0, int nx, int tid) {
+  if constexpr (W == 1) {
+    const int warp = tid >> 5, lane = tid & 31, i1 = lane + 32;
+    const int gx0 = s.gx[lane + B::OI + 1];
+    const int gx1 = i1 < B::NI ? s.gx[i1 + B::OI + 1] : 0;
+    const unsigned d0 = dst + 4u * (B::XO + lane);
+    for (int r = warp; r < B::NJ * B::NK; r += kThreads / 32) {
       const int j = r % B::NJ, k = r / B::NJ;
-      int xw = xs + 4 * v;  // a multiple of 4 in [-4, Sx + 35]: wrap into [0, Sx)
+      const float *row = src + (s.gz[k + B::OK + 1] + s.gy[j + B::OJ + 1]);
+      const unsigned d = d0 + 4u * (r * B::P);
+#pragma unroll
+      for (int f = 0; f < F; ++f) cp_async<1>(d + 4u * (f * B::N), row + gx0 + f * N);
+      if (i1 < B::NI) {
+#pragma unroll
+        for (int f = 0; f < F; ++f) cp_async<1>(d + 4u * (f * B::N + 32), row + gx1 + f * N);
+      }
+    }
+  } else {
+    constexpr int p0 = B::XO / W * W, PV = (B::XO + B::NI - p0 + W - 1) / W;
+    static_assert(p0 + W * PV <= B::P, "row length");
+    for (int e = tid; e < B::NJ * B::NK * PV; e += kThreads) {
+      const int r = e / PV, pos = p0 + W * (e - r * PV);
+      const int j = r % B::NJ, k = r / B::NJ;
+      int xw = x0 + B::OI - B::XO + pos;  // a multiple of W in [-4, Sx + 35]: wrap into [0, Sx)
       if (xw < 0) xw += nx;
       if (xw >= nx) xw %= nx;
       const float *p = src + (s.gz[k + B::OK + 1] + s.gy[j + B::OJ + 1] + xw);
-      const unsigned d = dst + 16u * (r * PV + v);
+      const unsigned d = dst + 4u * (r * B::P + pos);
 #pragma unroll
-      for (int f = 0; f < F; ++f) cp_async16(d + 4u * (f * B::N), p + f * N);
-    }
-    return;
-  }
-  const int warp = tid >> 5, lane = tid & 31, i1 = lane + 32;
-  const int gx0 = s.gx[lane + B::OI + 1];
-  const int gx1 = i1 < B::NI ? s.gx[i1 + B::OI + 1] : 0;
-  const unsigned d0 = dst + 4u * (B::XO + lane);
-  for (int r = warp; r < B::NJ * B::NK; r += kThreads / 32) {
-    const int j = r % B::NJ, k = r / B::NJ;
-    const float *row = src + (s.gz[k + B::OK + 1] + s.gy[j + B::OJ + 1]);
-    const unsigned d = d0 + 4u * (r * B::P);
-#pragma unroll
-    for (int f = 0; f < F; ++f) cp_async4(d + 4u * (f * B::N), row + gx0 + f * N);
-    if (i1 < B::NI) {
-#pragma unroll
-      for (int f = 0; f < F; ++f) cp_async4(d + 4u * (f * B::N + 32), row + gx1 + f * N);
+      for (int f = 0; f < F; ++f) cp_async<W>(d + 4u * (f * B::N), p + f * N);
     }
   }
+}
+
+// Every staged box of a tile: fields of the stage input, B fluxes, face B of
+// the step's state.
+template <int W>
+__device__ __forceinline__ void load_boxes(const Smem &s, unsigned vs, unsigned bs, unsigned ws,
+                                           const float *__restrict__ win, const float *__restrict__ wb,
+                                           const float *__restrict__ flux, size_t N, int x0, int nx, int tid) {
+  load_box<VelBox, 3, W>(s, vs, win + N, N, x0, nx, tid);
+  load_box<XYF, 1, W>(s, bs + 4 * kXY, flux + 5 * N, N, x0, nx, tid);
+  load_box<YXF, 1, W>(s, bs + 4 * kYX, flux + 13 * N, N, x0, nx, tid);
+  load_box<XZF, 1, W>(s, bs + 4 * kXZ, flux + 6 * N, N, x0, nx, tid);
+  load_box<ZXF, 1, W>(s, bs + 4 * kZX, flux + 19 * N, N, x0, nx, tid);
+  load_box<YZF, 1, W>(s, bs + 4 * kYZ, flux + 12 * N, N, x0, nx, tid);
+  load_box<ZYF, 1, W>(s, bs + 4 * kZY, flux + 20 * N, N, x0, nx, tid);
+  load_box<BXs, 1, W>(s, ws + 4 * fBX, wb + 5 * N, N, x0, nx, tid);
+  load_box<BYs, 1, W>(s, ws + 4 * fBY, wb + 6 * N, N, x0, nx, tid);
+  load_box<BZs, 1, W>(s, ws + 4 * fBZ, wb + 7 * N, N, x0, nx, tid);
 }
 
 // Corner EMFs (corner_magnet_flux, mhd_solver.inlrb:641-653) at the edges of
@@ -532,8 +549,9 @@ __device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, cons
   // Tiles whose staged rows and planes (y0-1..y0+4, z0-1..z0+2) lie inside the
   // box: one thread stages all of them with ten tensor copies; at an x edge
   // the copies leave zeros beyond it, and the one column there that is read is
-  // put in by single loads.  The others stage entry by entry through the
-  // wrapped offset tables (16-byte row chunks where rows are aligned).
+  // put in by single loads.  The others stage through the wrapped offset
+  // tables, in 16- or 8-byte row chunks where rows are aligned to them, else
+  // entry by entry.
   const bool tma = maps && maps->enabled && y0 >= 1 && y0 + 5 <= g.sy && z0 >= 1 && z0 + 3 <= g.sz;
   if (tma) {
     if (tid == 0) {
@@ -585,18 +603,9 @@ __device__ __forceinline__ void tile_epilogue(Smem &s, const GridParams &g, cons
       __syncthreads();
     }
   } else {
-    // whole 16-byte row chunks where rows are 16-byte aligned
-    const bool vec = (g.sx & 3) == 0;
-    load_box<VelBox, 3>(s, vs, win + N, N, x0, g.sx, vec, tid);
-    load_box<XYF, 1>(s, bs + 4 * kXY, flux + 5 * N, N, x0, g.sx, vec, tid);
-    load_box<YXF, 1>(s, bs + 4 * kYX, flux + 13 * N, N, x0, g.sx, vec, tid);
-    load_box<XZF, 1>(s, bs + 4 * kXZ, flux + 6 * N, N, x0, g.sx, vec, tid);
-    load_box<ZXF, 1>(s, bs + 4 * kZX, flux + 19 * N, N, x0, g.sx, vec, tid);
-    load_box<YZF, 1>(s, bs + 4 * kYZ, flux + 12 * N, N, x0, g.sx, vec, tid);
-    load_box<ZYF, 1>(s, bs + 4 * kZY, flux + 20 * N, N, x0, g.sx, vec, tid);
-    load_box<BXs, 1>(s, ws + 4 * fBX, wb + 5 * N, N, x0, g.sx, vec, tid);
-    load_box<BYs, 1>(s, ws + 4 * fBY, wb + 6 * N, N, x0, g.sx, vec, tid);
-    load_box<BZs, 1>(s, ws + 4 * fBZ, wb + 7 * N, N, x0, g.sx, vec, tid);
+    if ((g.sx & 3) == 0) load_boxes<4>(s, vs, bs, ws, win, wb, flux, N, x0, g.sx, tid);
+    else if ((g.sx & 1) == 0) load_boxes<2>(s, vs, bs, ws, win, wb, flux, N, x0, g.sx, tid);
+    else load_boxes<1>(s, vs, bs, ws, win, wb, flux, N, x0, g.sx, tid);
     cp_async_wait_all();
     __syncthreads();
   }

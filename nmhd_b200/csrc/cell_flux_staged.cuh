@@ -41,11 +41,33 @@ struct FluxMaps {
 // Shared index of tile-local cell (a, b, c).
 __device__ __forceinline__ int at(int a, int b, int c) { return ((c + 2) * NJ + (b + 2)) * P + XO + a; }
 
+// The staged rows by W-float asynchronous copies (Sx % W == 0), the tile's
+// threads over all (row, chunk) pairs of the positions that are read
+// (x0-2..x0+32); a chunk beyond an x edge of the box is the (still aligned)
+// chunk Sx away.  A flux launch of a 250x97x61 box took 169 us with 4-byte
+// copies a row to a warp, 142 us so; of a 251x97x61 box 156 us.
+template <int W>
+__device__ __forceinline__ void copy_rows(const Smem &s, int nx, const float *__restrict__ w, size_t N, unsigned ds,
+                                          int x0, int tid) {
+  constexpr int p0 = 2 / W * W, PV = (37 - p0 + W - 1) / W;
+  static_assert(p0 + W * PV <= P, "row length");
+  for (int e = tid; e < NJ * NK * PV; e += kThreads) {
+    const int r = e / PV, pos = p0 + W * (e - r * PV);
+    int xw = x0 - XO + pos;  // a multiple of W in [-4, Sx + 35]: wrap into [0, Sx)
+    if (xw < 0) xw += nx;
+    if (xw >= nx) xw %= nx;
+    const float *src = w + (s.gz[r / NJ] + s.gy[r % NJ] + xw);
+    const unsigned d = ds + 4u * (r * P + pos);
+#pragma unroll
+    for (int f = 0; f < 8; ++f) epi::cp_async<W>(d + 4u * (f * FS), src + f * N);
+  }
+}
+
 // Copies the stage input w around tile (x0, y0, z0) into s.w.  Tiles whose box
 // lies inside the grid: one tensor copy issued by thread 0, completing on the
 // mbarrier (bounded wait; false if it timed out).  Others: cp.async through
-// the wrapped offset tables, 16-byte row chunks where Sx % 4 == 0, else entry
-// by entry.  Every thread of the CTA calls it.  kOnce: the CTA stages no other
+// the wrapped offset tables, in the widest row chunks that Sx is a multiple of
+// (16, 8 or 4 bytes).  Every thread of the CTA calls it.  kOnce: the CTA stages no other
 // tile, so a thread goes on when it has seen the copy land (and the answer is
 // the thread's own).
 template <bool kOnce = false>
@@ -88,36 +110,9 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
   else if (tid < P + NJ) s.gy[tid - P] = wrap_any(y0 - 2 + (tid - P), g.sy) * g.sx;
   else if (tid < P + NJ + NK) s.gz[tid - P - NJ] = wrap_any(z0 - 2 + (tid - P - NJ), g.sz) * g.sx * g.sy;
   __syncthreads();
-  constexpr int R = NJ * NK;
-  if ((g.sx & 3) == 0) {
-    // 16-byte chunks of the rows; a chunk beyond an x edge of the box is the
-    // (aligned) chunk Sx away
-    constexpr int PV = P / 4;
-    const int xs = x0 - XO;
-    for (int e = tid; e < R * PV; e += kThreads) {
-      const int r = e / PV, v = e - r * PV;
-      int xw = xs + 4 * v;  // a multiple of 4 in [-4, Sx + 35]: wrap into [0, Sx)
-      if (xw < 0) xw += g.sx;
-      if (xw >= g.sx) xw %= g.sx;
-      const float *src = w + (s.gz[r / NJ] + s.gy[r % NJ] + xw);
-      const unsigned d = ds + 16u * (r * PV + v);
-#pragma unroll
-      for (int f = 0; f < 8; ++f) epi::cp_async16(d + 4u * (f * FS), src + f * N);
-    }
-  } else {
-    // one row per warp at a time: lanes 0-31 and 0-7 again for entries 32-39
-    const int warp = tid >> 5, lane = tid & 31;
-    const int gx0 = s.gx[lane], gx1 = lane < P - 32 ? s.gx[lane + 32] : 0;
-    for (int r = warp; r < R; r += kThreads / 32) {
-      const float *row = w + (s.gz[r / NJ] + s.gy[r % NJ]);
-      const unsigned d = ds + 4u * (r * P + lane);
-#pragma unroll
-      for (int f = 0; f < 8; ++f) {
-        epi::cp_async4(d + 4u * (f * FS), row + gx0 + f * N);
-        if (lane < P - 32) epi::cp_async4(d + 4u * (f * FS + 32), row + gx1 + f * N);
-      }
-    }
-  }
+  if ((g.sx & 3) == 0) copy_rows<4>(s, g.sx, w, N, ds, x0, tid);
+  else if ((g.sx & 1) == 0) copy_rows<2>(s, g.sx, w, N, ds, x0, tid);
+  else copy_rows<1>(s, g.sx, w, N, ds, x0, tid);
   epi::cp_async_wait_all();
   __syncthreads();
   return true;
