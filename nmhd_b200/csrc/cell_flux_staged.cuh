@@ -8,9 +8,10 @@
 // copies all 8 fields of the cells x0-2..x0+32, y0-2..y0+4, z0-2..z0+2 (the
 // union of the three axes' 4-cell stencils and the +1 transverse neighbours
 // of the face-centred B) into shared memory, with one tensor copy for tiles
-// away from the box edges; every stencil read is then a shared load at a
-// constant or axis-stride offset.  The arithmetic is face_flux()'s, the same
-// code the per-cell kernel runs, so the fluxes are bitwise the same.
+// away from the box's y and z edges; every stencil read is then a shared load
+// at a constant offset.  The fluxes are bitwise face_flux()'s: the quotients
+// and roots are correctly rounded in both, here by shared reciprocals where the
+// operands are in their range (rounded.cuh), else by the plain operations.
 #pragma once
 #include "cell_epilogue.cuh"
 
@@ -63,9 +64,30 @@ __device__ __forceinline__ void copy_rows(const Smem &s, int nx, const float *__
   }
 }
 
-// Copies the stage input w around tile (x0, y0, z0) into s.w.  Tiles whose box
-// lies inside the grid: one tensor copy issued by thread 0, completing on the
-// mbarrier (bounded wait; false if it timed out).  Others: cp.async through
+// What staged row e (field, z, y) holds beyond the x edges of the box: cells
+// Sx-2 and Sx-1 before the first column, cell 0 after the last.  Of tiles whose
+// rows and planes lie inside the box.
+constexpr int kRows = 8 * NJ * NK;
+static_assert(kRows <= 2 * kThreads, "two rows a thread");
+struct Wrapped {
+  float l2, l1, h;
+};
+__device__ __forceinline__ Wrapped wrapped_columns(const GridParams &g, const float *__restrict__ w, bool low,
+                                                   bool high, int y0, int z0, int e) {
+  const int f = e / (NJ * NK), r = e - f * (NJ * NK);
+  const float *row = w + f * (size_t)g.n + ((z0 - 2 + r / NJ) * g.sy + (y0 - 2 + r % NJ)) * g.sx;
+  Wrapped v = {};
+  if (low) v.l2 = __ldg(row + g.sx - 2), v.l1 = __ldg(row + g.sx - 1);
+  if (high) v.h = __ldg(row);
+  return v;
+}
+
+// Copies the stage input w around tile (x0, y0, z0) into s.w.  Tiles whose rows
+// and planes lie inside the box: one tensor copy issued by thread 0, completing
+// on the mbarrier (bounded wait; false if it timed out); beyond an x edge it
+// leaves zeros, and the columns there that are read are put in by single loads
+// (tiles at x edges by 16-byte copies: 162 us a launch on the 256x128x64 box, so
+// 156; 31.2 -> 29.2 us on 64^3, where every tile is at one).  Others: cp.async through
 // the wrapped offset tables, in the widest row chunks that Sx is a multiple of
 // (16, 8 or 4 bytes).  Every thread of the CTA calls it.  kOnce: the CTA stages no other
 // tile, so a thread goes on when it has seen the copy land (and the answer is
@@ -75,9 +97,26 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
                                       const float *__restrict__ w, int x0, int y0, int z0, int tid) {
   const size_t N = (size_t)g.n;
   const unsigned ds = (unsigned)__cvta_generic_to_shared(s.w), mb = (unsigned)__cvta_generic_to_shared(&s.mbar);
-  const bool tma = maps && maps->enabled && x0 >= 4 && x0 + 36 <= g.sx && y0 >= 2 && y0 + 5 <= g.sy && z0 >= 2 &&
-                   z0 + 3 <= g.sz;
+  const bool tma = maps && maps->enabled && y0 >= 2 && y0 + 5 <= g.sy && z0 >= 2 && z0 + 3 <= g.sz;
   if (tma) {
+    const bool low = x0 == 0, high = x0 + BX >= g.sx;
+    Wrapped wr[2];
+    if (low || high) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (tid + i * kThreads < kRows) wr[i] = wrapped_columns(g, w, low, high, y0, z0, tid + i * kThreads);
+    }
+    auto patch = [&] {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int e = tid + i * kThreads;
+        if (e >= kRows) break;
+        float *row = s.w + e * P + XO;
+        if (low) row[-2] = wr[i].l2, row[-1] = wr[i].l1;
+        if (high) row[g.sx - x0] = wr[i].h;
+      }
+      __syncthreads();
+    };
     if (tid == 0) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -93,7 +132,11 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
     __syncthreads();
     // (a second bounded wait where the first gives up: no copy may still be
     // writing when the CTA exits)
-    if (kOnce) return epi::mbar_wait_bounded(mb) || (epi::mbar_wait_bounded(mb), false);
+    if (kOnce) {
+      const bool ok = epi::mbar_wait_bounded(mb) || (epi::mbar_wait_bounded(mb), false);
+      if (low || high) patch();
+      return ok;
+    }
     const bool ok = __syncthreads_and(epi::mbar_wait_bounded(mb));
     if (!ok) {
       // flag it and wait once more (bounded) so that no copy is still
@@ -104,6 +147,7 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
       return false;
     }
     if (tid == 0) asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(mb) : "memory");
+    if (low || high) patch();
     return true;
   }
   if (tid < P) s.gx[tid] = wrap_any(x0 - XO + tid, g.sx);
@@ -187,7 +231,7 @@ static __device__ __noinline__ void plain_face(const GridParams &g, const float 
 // one Riemann solver (three overflow the instruction caches) and a branch per
 // axis that reads its input: with the axis a run-time number in the input too,
 // a tenth of the instructions made addresses.  256x128x64 box: 1,912 warp
-// instructions for a warp's three faces (2,293 before), 163 us a launch (181),
+// instructions for a warp's three faces (2,293 before), 162 us a launch (181),
 // 72 % of the issue slots filled.  Four CTAs/SM hide the start and the staging
 // of a tile better than one persistent CTA of 1,024 threads with a ring of five
 // copies (201 us: its spills miss the small L1 that is left) or a stagger of

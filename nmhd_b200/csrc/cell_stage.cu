@@ -51,7 +51,8 @@
 #define NMHD_EPI_MIN_BLOCKS (kPow2 ? 5 : 4)
 #endif
 // The staged flux kernel holds 44 KB of shared memory per CTA: 4 CTAs/SM, 163 us
-// a launch on the 256x128x64 box (3: 165, 5: 168).
+// a launch on the 256x128x64 box (3: 165, 5: 168; 156 at 4 now that the tiles
+// at x edges are staged by tensor copies too).
 #ifndef NMHD_SFLUX_MIN_BLOCKS
 #define NMHD_SFLUX_MIN_BLOCKS 4
 #endif
