@@ -162,13 +162,39 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
   return true;
 }
 
+// The states on either side of a face from the cells' values x0..x3, and from
+// sums of two values, which halve exactly where q.slope() holds.
+template <class Q>
+__device__ __forceinline__ void face_states(Q &q, const float x[4], float &l, float &r) {
+  reconstruct4_with(q, x[0], x[1], x[2], x[3], l, r);
+}
+template <class Q>
+__device__ __forceinline__ void face_means(Q &q, const float s[4], float &l, float &r) {
+  reconstruct4_with(q, s[0], s[1], s[2], s[3], l, r);
+  l *= 0.5f;
+  r *= 0.5f;
+}
+#if NMHD_FAST_ARITH
+// The fast-arithmetic kernel keeps face_input()'s and hlld_flux_plain()'s
+// operations as they stand.  With products by shared approximate reciprocals
+// and the three-instruction limiter a launch took 122 us instead of 141
+// (256x128x64 box), but after 16 steps the state was off the FP64 one by 5.3e-4
+// instead of 4.6e-4.
+struct AsCompiled {};
+__device__ __forceinline__ void face_states(AsCompiled, const float x[4], float &l, float &r) {
+  reconstruct4(x[0], x[1], x[2], x[3], l, r);
+}
+__device__ __forceinline__ void face_means(AsCompiled, const float s[4], float &l, float &r) {
+  reconstruct4(0.5f * s[0], 0.5f * s[1], 0.5f * s[2], 0.5f * s[3], l, r);
+}
+#endif
+
 // face_input() from the shared copy for the lower AX-face of cell index ci, in
 // the arithmetic Q.  With the axis a constant every shared read is at a
-// constant offset from the cell's address.  Transverse B is reconstructed from
-// the sums of the two faces, which halve exactly where q.slope() holds.
-template <int AX, bool kOrder2, class Q>
-__device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, const float *w, int ci, int yidx,
-                                               float half_dt) {
+// constant offset from the cell's address.
+template <int AX, class Q>
+__device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, bool order2, const float *w, int ci,
+                                               int yidx, float half_dt) {
   constexpr int E1 = (AX + 1) % 3, E2 = (AX + 2) % 3;
   constexpr int stride[3] = {1, DY, DZ};
   constexpr int sa = stride[AX], t1 = stride[E1], t2 = stride[E2];
@@ -178,23 +204,26 @@ __device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, const 
   // 0 or far above the least and need no check
   auto pair = [&](int f, auto &&checks, float &l, float &r) {
     const float *p = c + f * FS;
-    if constexpr (kOrder2) reconstruct4_with(checks, p[-2 * sa], p[-sa], p[0], p[sa], l, r);
-    else l = p[-sa], r = p[0];
+    const float x[4] = {p[-2 * sa], p[-sa], p[0], p[sa]};
+    if (order2) face_states(checks, x, l, r);
+    else l = x[1], r = x[2];
   };
   auto field = [&](int f, int t, float &l, float &r) {
     const float *p = c + f * FS;
-    if constexpr (kOrder2)
-      reconstruct4_with(q, p[-2 * sa] + p[t - 2 * sa], p[-sa] + p[t - sa], p[0] + p[t], p[sa] + p[t + sa], l, r);
-    else
-      l = p[-sa] + p[t - sa], r = p[0] + p[t];
-    l *= 0.5f;
-    r *= 0.5f;
+    const float s[4] = {p[-2 * sa] + p[t - 2 * sa], p[-sa] + p[t - sa], p[0] + p[t], p[sa] + p[t + sa]};
+    if (order2) face_means(q, s, l, r);
+    else l = 0.5f * s[1], r = 0.5f * s[2];
   };
-  pair(0, Ieee(), in.dl, in.dr);
+#if NMHD_FAST_ARITH
+  Q &unchecked = q;
+#else
+  Ieee unchecked;
+#endif
+  pair(0, unchecked, in.dl, in.dr);
   pair(1 + AX, q, in.ul, in.ur);
   pair(1 + E1, q, in.vl, in.vr);
   pair(1 + E2, q, in.wl, in.wr);
-  pair(4, Ieee(), in.pl, in.pr);
+  pair(4, unchecked, in.pl, in.pr);
   field(5 + E1, t1, in.byl, in.byr);
   field(5 + E2, t2, in.bzl, in.bzr);
   if (AX < 2 && g.shear) {
@@ -203,8 +232,16 @@ __device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, const 
     const float *p = c + (AX == 0 ? 2 : 1) * FS;
     const float v = 0.5f * (p[-sa] + p[0]);
     float acc;
-    if (AX == 0) acc = -2.0f * g.omega * v;
-    else acc = 2.0f * g.omega * v + 2.0f * g.q * (g.omega * g.omega) * (g.corner_y + g.dy * ((float)yidx + 0.5f));
+    if (AX == 0) {
+      acc = -2.0f * g.omega * v;
+    } else {
+      const float tide = 2.0f * g.q * (g.omega * g.omega), at = g.corner_y + g.dy * ((float)yidx + 0.5f);
+#if NMHD_FAST_ARITH
+      acc = fmaf(tide, at, 2.0f * g.omega * v);  // contracted so, whatever the compiler would choose
+#else
+      acc = 2.0f * g.omega * v + tide * at;
+#endif
+    }
     const float mbv = half_dt * acc;
     in.ul += mbv;
     in.ur += mbv;
@@ -236,8 +273,7 @@ static __device__ __noinline__ void plain_face(const GridParams &g, const float 
 // of a tile better than one persistent CTA of 1,024 threads with a ring of five
 // copies (201 us: its spills miss the small L1 that is left) or a stagger of
 // the first CTAs (172 us).
-template <bool kOrder2>
-__device__ __forceinline__ void flux_cell_order(const GridParams &g, const float *w, float *__restrict__ flux, int ci,
+__device__ __forceinline__ void flux_cell_order(const GridParams &g, bool order2, const float *w, float *__restrict__ flux, int ci,
                                                 unsigned o, int y, float dt, int ax0, int ax1) {
   const size_t N = (size_t)g.n;
   const float half_dt = 0.5f * dt;
@@ -247,17 +283,20 @@ __device__ __forceinline__ void flux_cell_order(const GridParams &g, const float
     char *base = reinterpret_cast<char *>(flux + (size_t)(7 * ax) * N);
     auto out = [&](int k, float v) { *reinterpret_cast<float *>(base + k * (4 * N) + 4u * o) = v; };
 #if NMHD_FAST_ARITH
-    Approximate q;
+    AsCompiled q;
 #else
     Ranged q;
 #endif
     const float bn = w[(5 + ax) * FS + ci];
     HlldIn in;
-    if (ax == 0) in = staged_input<0, kOrder2>(q, g, w, ci, y, half_dt);
-    else if (ax == 1) in = staged_input<1, kOrder2>(q, g, w, ci, y, half_dt);
-    else in = staged_input<2, kOrder2>(q, g, w, ci, y, half_dt);
+    if (ax == 0) in = staged_input<0>(q, g, order2, w, ci, y, half_dt);
+    else if (ax == 1) in = staged_input<1>(q, g, order2, w, ci, y, half_dt);
+    else in = staged_input<2>(q, g, order2, w, ci, y, half_dt);
 #if NMHD_FAST_ARITH
-    hlld_flux_with(q, g.gamma, Approximate::under(g.gamma - 1.0f), bn, in, out);
+    float f[7];
+    hlld_flux_plain(g.gamma, bn, in, f);
+#pragma unroll
+    for (int k = 0; k < 7; ++k) out(k, f[k]);
 #else
     const bool ok = hlld_flux_with(q, g.gamma, g.gm1, bn, in, out);
     if (!(ok && g.ranged)) plain_face(g, w, flux, ci, ax, (int)o, y, half_dt);
@@ -269,8 +308,13 @@ __device__ __forceinline__ void flux_cell_staged(const GridParams &g, const floa
                                                  int a, int b, int c, int x, int y, int z, float dt, int ax0 = 0,
                                                  int ax1 = 3) {
   const unsigned o = (unsigned)((z * g.sy + y) * g.sx + x);
-  if (g.order2) flux_cell_order<true>(g, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
-  else flux_cell_order<false>(g, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
+#if NMHD_FAST_ARITH
+  flux_cell_order(g, g.order2, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
+#else
+  // the order a constant in each of two copies of the code
+  if (g.order2) flux_cell_order(g, true, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
+  else flux_cell_order(g, false, w, flux, at(a, b, c), o, y, dt, ax0, ax1);
+#endif
 }
 
 }  // namespace sfx

@@ -7,9 +7,9 @@
 // root (-prec-div=true, -prec-sqrt=true, no flush-to-zero) are the defaults.
 //
 // With NMHD_FAST_ARITH (the fast-arithmetic flux kernel, cell_fast.cu, compiled
-// with contraction and approximate square root) hlld_flux_with<Approximate>
-// evaluates the energy in float: results within the documented tolerance of
-// the reference instead of bitwise.
+// with contraction and approximate division and square root) the FP64
+// sub-expressions of hlld_flux_plain() are evaluated in float: results within
+// the documented tolerance of the reference instead of bitwise.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -99,11 +99,16 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   const float B2_R = B2x + By_R * By_R + Bz_R * Bz_R;
   const float v2_R = velx_R * velx_R + vely_R * vely_R + velz_R * velz_R;
   const float gm1 = gamma - 1.0f;
+#if NMHD_FAST_ARITH
+  const float etot_L = pres_L / gm1 + 0.5f * dens_L * v2_L + 0.5f * B2_L;
+  const float etot_R = pres_R / gm1 + 0.5f * dens_R * v2_R + 0.5f * B2_R;
+#else
   // etot = p/(gamma-1) + 0.5*rho*v2 + 0.5*B2, the last two terms in double
   const float etot_L = (float)((double)(pres_L / gm1) + 0.5 * (double)dens_L * (double)v2_L +
                                0.5 * (double)B2_L);
   const float etot_R = (float)((double)(pres_R / gm1) + 0.5 * (double)dens_R * (double)v2_R +
                                0.5 * (double)B2_R);
+#endif
 
   const float gpl = gamma * pres_L, gpr = gamma * pres_R;
   const float gpbl = gpl + B2_L, gpbr = gpr + B2_R;
@@ -115,6 +120,14 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   const float S_L = fminf(velx_L, velx_R) - cfmax;
   const float S_R = fmaxf(velx_L, velx_R) + cfmax;
 
+#if NMHD_FAST_ARITH
+  const float pT_L = pres_L + 0.5f * B2_L;
+  const float pT_R = pres_R + 0.5f * B2_R;
+  const float sRv = S_R - velx_R, sLv = S_L - velx_L;
+  const float rden = 1.0f / (sRv * dens_R - sLv * dens_L);
+  const float S_M = (sRv * momx_R - sLv * momx_L - pT_R + pT_L) * rden;
+  const float pT_s = (sRv * dens_R * pT_L - sLv * dens_L * pT_R + dens_L * dens_R * sRv * sLv * (velx_R - velx_L)) * rden;
+#else
   // p + 0.5*B2: exact 0.5*B2 in double, one double add, rounded to float
   const float pT_L = (float)((double)pres_L + 0.5 * (double)B2_L);
   const float pT_R = (float)((double)pres_R + 0.5 * (double)B2_R);
@@ -127,6 +140,7 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
   float pT_s = sRv * dens_R * pT_L - sLv * dens_L * pT_R;
   pT_s = pT_s + dens_L * dens_R * sRv * sLv * (velx_R - velx_L);
   pT_s = (float)((double)pT_s * rden);
+#endif
 
   const float sLm = S_L - S_M, sRm = S_R - S_M;
   // Single-star densities of both sides fix the Alfven speeds S_L*, S_R*
@@ -261,8 +275,7 @@ __host__ __device__ __forceinline__ void hlld_flux_plain(const float gamma, cons
 //  - 0.5 * d * v2 and 0.5 * B2 are exact in double, so adding each with a
 //    fused multiply-add rounds where the separate addition did.
 // gm1: gamma - 1 as a denominator.  A is the arithmetic of its quotients and
-// roots: Ranged here, Approximate (which tests no range) in the fast-arithmetic
-// kernel, where the energy's sums are in float as in the rest of that kernel.
+// roots (Ranged).
 // out(k, v) takes flux k; it is called in each branch of the fan, where the
 // caller can store the values at once: as results of the branches they cost a
 // move each at every join.
@@ -334,11 +347,7 @@ __host__ __device__ __forceinline__ bool hlld_flux_with(A &q, const float gamma,
 
   const float v2_ = u_ * u_ + v_ * v_ + w_ * w_;
   const float heat = q.ratio(p_, gm1);
-#if NMHD_FAST_ARITH
-  const float e_ = heat + 0.5f * d_ * v2_ + 0.5f * B2_;
-#else
   const float e_ = (float)fma(0.5, (double)B2_, fma(0.5, (double)d_ * (double)v2_, (double)heat));
-#endif
   const float vB_ = u_ * Bx + v_ * by_ + w_ * bz_;
   const float mx_ = d_ * u_, my_ = d_ * v_, mz_ = d_ * w_;
   const float Bby = Bx * by_, Bbz = Bx * bz_;

@@ -146,17 +146,4 @@ struct Ieee {
   __host__ __device__ __forceinline__ static bool hold() { return true; }
 };
 
-// Products with approximate reciprocals (within 2 ulp), for the opt-in fast
-// arithmetic.
-struct Approximate {
-  __device__ __forceinline__ static void positive(float) {}
-  __device__ __forceinline__ static void slope(float) {}
-  __device__ __forceinline__ static Denominator under(float b) { return Denominator{b, approx_inverse(b)}; }
-  __device__ __forceinline__ static float ratio(float a, const Denominator &d) { return a * d.h; }
-  __device__ __forceinline__ static float div(float a, const Denominator &d) { return a * d.h; }
-  __device__ __forceinline__ static float div_bounded(float a, const Denominator &d) { return a * d.h; }
-  __device__ __forceinline__ static float root(float x) { return sqrtf(x); }
-  __device__ __forceinline__ static bool hold() { return true; }
-};
-
 }  // namespace nmhd
