@@ -188,15 +188,12 @@ __device__ __forceinline__ void load_box(const Smem &s, unsigned dst, const floa
       }
     }
   } else {
-    constexpr int p0 = B::XO / W * W, PV = (B::XO + B::NI - p0 + W - 1) / W;
-    static_assert(p0 + W * PV <= B::P, "row length");
-    for (int e = tid; e < B::NJ * B::NK * PV; e += kThreads) {
-      const int r = e / PV, pos = p0 + W * (e - r * PV);
+    using Chunks = RowChunks<B::XO, B::XO + B::NI, W>;
+    static_assert(Chunks::first + W * Chunks::count <= B::P, "row length");
+    for (int e = tid; e < B::NJ * B::NK * Chunks::count; e += kThreads) {
+      const int r = e / Chunks::count, pos = Chunks::first + W * (e - r * Chunks::count);
       const int j = r % B::NJ, k = r / B::NJ;
-      int xw = x0 + B::OI - B::XO + pos;  // a multiple of W in [-4, Sx + 35]: wrap into [0, Sx)
-      if (xw < 0) xw += nx;
-      if (xw >= nx) xw %= nx;
-      const float *p = src + (s.gz[k + B::OK + 1] + s.gy[j + B::OJ + 1] + xw);
+      const float *p = src + (s.gz[k + B::OK + 1] + s.gy[j + B::OJ + 1] + row_column<W>(x0 + B::OI - B::XO + pos, nx));
       const unsigned d = dst + 4u * (r * B::P + pos);
 #pragma unroll
       for (int f = 0; f < F; ++f) cp_async<W>(d + 4u * (f * B::N), p + f * N);

@@ -23,12 +23,13 @@ namespace sfx {
 // (x0 at row position 4), NJ = 7 rows (y0-2..y0+4) per plane, NK = 5 planes
 // (z0-2..z0+2), the 8 fields FS floats apart.
 constexpr int P = 40, NJ = 7, NK = 5, XO = 4;
+constexpr int kReadBegin = XO - 2, kReadEnd = XO + BX + 1;  // row positions that are read (x0-2..x0+32)
 constexpr int DY = P, DZ = P * NJ, FS = P * NJ * NK;
 constexpr unsigned kTxBytes = 4u * 8u * FS;
 
 struct __align__(128) Smem {
   float w[8 * FS];
-  int gx[P], gy[NJ], gz[NK];  // wrapped global offsets of x0-4+i, (y0-2+j)*Sx, (z0-2+k)*Sx*Sy
+  int gy[NJ], gz[NK];  // wrapped global offsets of (y0-2+j)*Sx, (z0-2+k)*Sx*Sy
   unsigned long long mbar;
 };
 
@@ -50,14 +51,11 @@ __device__ __forceinline__ int at(int a, int b, int c) { return ((c + 2) * NJ + 
 template <int W>
 __device__ __forceinline__ void copy_rows(const Smem &s, int nx, const float *__restrict__ w, size_t N, unsigned ds,
                                           int x0, int tid) {
-  constexpr int p0 = 2 / W * W, PV = (37 - p0 + W - 1) / W;
-  static_assert(p0 + W * PV <= P, "row length");
-  for (int e = tid; e < NJ * NK * PV; e += kThreads) {
-    const int r = e / PV, pos = p0 + W * (e - r * PV);
-    int xw = x0 - XO + pos;  // a multiple of W in [-4, Sx + 35]: wrap into [0, Sx)
-    if (xw < 0) xw += nx;
-    if (xw >= nx) xw %= nx;
-    const float *src = w + (s.gz[r / NJ] + s.gy[r % NJ] + xw);
+  using Chunks = RowChunks<kReadBegin, kReadEnd, W>;
+  static_assert(Chunks::first + W * Chunks::count <= P, "row length");
+  for (int e = tid; e < NJ * NK * Chunks::count; e += kThreads) {
+    const int r = e / Chunks::count, pos = Chunks::first + W * (e - r * Chunks::count);
+    const float *src = w + (s.gz[r / NJ] + s.gy[r % NJ] + row_column<W>(x0 - XO + pos, nx));
     const unsigned d = ds + 4u * (r * P + pos);
 #pragma unroll
     for (int f = 0; f < 8; ++f) epi::cp_async<W>(d + 4u * (f * FS), src + f * N);
@@ -150,9 +148,8 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
     if (low || high) patch();
     return true;
   }
-  if (tid < P) s.gx[tid] = wrap_any(x0 - XO + tid, g.sx);
-  else if (tid < P + NJ) s.gy[tid - P] = wrap_any(y0 - 2 + (tid - P), g.sy) * g.sx;
-  else if (tid < P + NJ + NK) s.gz[tid - P - NJ] = wrap_any(z0 - 2 + (tid - P - NJ), g.sz) * g.sx * g.sy;
+  if (tid < NJ) s.gy[tid] = wrap_any(y0 - 2 + tid, g.sy) * g.sx;
+  else if (tid < NJ + NK) s.gz[tid - NJ] = wrap_any(z0 - 2 + (tid - NJ), g.sz) * g.sx * g.sy;
   __syncthreads();
   if ((g.sx & 3) == 0) copy_rows<4>(s, g.sx, w, N, ds, x0, tid);
   else if ((g.sx & 1) == 0) copy_rows<2>(s, g.sx, w, N, ds, x0, tid);

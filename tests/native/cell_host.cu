@@ -5,7 +5,7 @@
 // and double operation separately (-ffp-contract=off, SSE arithmetic), so the
 // results are the device's and the tests can compare them bitwise with the
 // oracle on a CPU.  Not part of the library; nothing in nmhd_b200 loads it.
-#include "../../nmhd_b200/csrc/mhd_math.cuh"
+#include "../../nmhd_b200/csrc/cell_flux_staged.cuh"
 
 extern "C" {
 
@@ -49,3 +49,46 @@ void cellh_reconstruct_ranged_f32(const float *x, float *lr, int *ok, long n) {
 }
 
 }  // extern "C"
+
+// The columns of a box nx cells wide that the staging of a tile at x0 copies into
+// a row of one of its boxes (0: the flux kernel's, 1..: the update kernel's), in
+// chunks of W floats: out[position - origin], -1 where nothing is copied;
+// `inside` false where a chunk leaves the row of the box.  Row position p stands
+// for x0 + *origin + p; positions [*begin, *end) are read.
+namespace {
+template <int kBegin, int kEnd, int W>
+int copied(int x0, int origin, int nx, int *out) {
+  using C = nmhd::cell::RowChunks<kBegin, kEnd, W>;
+  int inside = 1;
+  for (int c = 0; c < C::count; ++c) {
+    const int pos = C::first + W * c, col = nmhd::cell::row_column<W>(x0 + origin + pos, nx);
+    inside = inside && col >= 0 && col + W <= nx;
+    for (int i = 0; i < W; ++i) out[pos + i] = col + i;
+  }
+  return inside;
+}
+template <int kBegin, int kEnd>
+int copied(int W, int x0, int o, int nx, int *out, int *origin, int *begin, int *end) {
+  *origin = o, *begin = kBegin, *end = kEnd;
+  return W == 4   ? copied<kBegin, kEnd, 4>(x0, o, nx, out)
+         : W == 2 ? copied<kBegin, kEnd, 2>(x0, o, nx, out)
+                  : copied<kBegin, kEnd, 1>(x0, o, nx, out);
+}
+template <class B>
+int copied_box(int W, int x0, int nx, int *out, int *origin, int *begin, int *end) {
+  return copied<B::XO, B::XO + B::NI>(W, x0, B::OI - B::XO, nx, out, origin, begin, end);
+}
+}  // namespace
+
+extern "C" int cellh_staged_columns(int box, int W, int x0, int nx, int *out, int *origin, int *begin, int *end) {
+  using namespace nmhd::cell;
+  for (int i = 0; i < 40; ++i) out[i] = -1;
+  switch (box) {
+    case 0: return copied<sfx::kReadBegin, sfx::kReadEnd>(W, x0, -sfx::XO, nx, out, origin, begin, end);
+    case 1: return copied_box<epi::VelBox>(W, x0, nx, out, origin, begin, end);
+    case 2: return copied_box<epi::XYF>(W, x0, nx, out, origin, begin, end);
+    case 3: return copied_box<epi::YXF>(W, x0, nx, out, origin, begin, end);
+    case 4: return copied_box<epi::ZYF>(W, x0, nx, out, origin, begin, end);
+    default: return -1;
+  }
+}

@@ -88,6 +88,25 @@ def test_batch_boxes_equal_single_box_runs(gpu, schedule):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("persistent", [False, True])
+def test_batch_of_narrow_boxes_in_the_staged_passes(gpu, persistent):
+    """Boxes 1 to 5 cells wide in x, whose staged rows wrap more than once."""
+    from nmhd_b200.batch import BatchSolver
+    from nmhd_b200.solver import MHDSolver
+    boxes = [orszag_tang_3d(n, ny=9, nz=6) for n in (1, 2, 3, 4, 5)] + [orszag_tang_3d(1, ny=1, nz=1)]
+    with BatchSolver([c for c, _ in boxes]) as batch:
+        for k in range(5):
+            batch.set_schedule(k, persistent, True)
+        batch.set_states([s for _, s in boxes])
+        batch.step(3)
+        for i, (c, s) in enumerate(boxes):
+            with MHDSolver(c) as one:
+                one.set_state(s)
+                one.step(3)
+                assert np.array_equal(batch.get_state(i), one.get_state()), f"box {i}"
+
+
+@pytest.mark.gpu
 def test_batch_goal_time_per_box(gpu):
     """Per-box goal times, with the batch on a caller's stream."""
     import torch

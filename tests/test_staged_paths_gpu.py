@@ -1,6 +1,6 @@
 """The staged kernels at the row lengths and value ranges where their paths
 part: rows that are multiples of 4, 2 and 1 floats with a partial tile at the x
-edge, and units that put density, pressure or slopes outside the range that the
+edge, down to one cell, and units that put density, pressure or slopes outside the range that the
 shared reciprocals cover, everywhere or in some cells only, so that those faces
 and quotients take the plain arithmetic.  Bitwise the oracle: one scheme, each
 operation rounded the same."""
@@ -15,7 +15,7 @@ from test_parity_gpu import assert_same, run_gpu
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(6, 5, 3), (34, 13, 7), (35, 13, 7), (36, 13, 7), (37, 9, 5), (64, 16, 8), (70, 18, 6),
+@pytest.mark.parametrize("nx,ny,nz", [(1, 5, 3), (2, 13, 7), (3, 5, 3), (4, 13, 7), (6, 5, 3), (34, 13, 7), (35, 13, 7), (36, 13, 7), (37, 9, 5), (64, 16, 8), (70, 18, 6),
                                       (100, 14, 6)])
 @pytest.mark.parametrize("units", ["plain", "light", "light_mixed", "dense_mixed", "still"])
 def test_staged_paths_match_oracle(gpu, nx, ny, nz, units):

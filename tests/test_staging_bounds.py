@@ -13,8 +13,14 @@ holds the cell the reference's periodic neighbour offsets name.
 Fused epilogue: the staged boxes cover every cell, edge and face its phases
 read (corner EMFs of the tile and its upper halo edges, new face B, the
 cell update's lower and upper faces)."""
+import ctypes
 import os
 import re
+
+import numpy as np
+import pytest
+
+from test_face_math_cpu import lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "..", "nmhd_b200", "csrc")
@@ -31,9 +37,9 @@ def sfx_constants():
     assert m, "staged box constants not found"
     P, NJ, NK, XO = map(int, m.groups())
     # the box origin relative to the tile: x0 - XO, y0 - 2, z0 - 2 (tensor copy
-    # coordinates and the wrapped offset tables)
+    # coordinates, row chunks and the wrapped offset tables)
     assert '"r"(x0 - XO), "r"(y0 - 2), "r"(z0 - 2)' in t
-    assert "wrap_any(x0 - XO + tid, g.sx)" in t and "wrap_any(y0 - 2 + (tid - P), g.sy)" in t
+    assert "row_column<W>(x0 - XO + pos, nx)" in t and "wrap_any(y0 - 2 + tid, g.sy)" in t
     assert re.search(r"return \(\(c \+ 2\) \* NJ \+ \(b \+ 2\)\) \* P \+ XO \+ a;", t), "at() changed"
     return P, NJ, NK, XO
 
@@ -134,3 +140,26 @@ def test_epilogue_boxes_cover_every_read():
                 assert covers(B["BZs"], a, b, c)
                 assert covers(B["YEdge"], a, b, c) and covers(B["YEdge"], a + 1, b, c)
                 assert covers(B["XEdge"], a, b, c) and covers(B["XEdge"], a, b + 1, c)
+
+
+@pytest.mark.parametrize("box", range(5))
+def test_row_chunks_hold_the_periodic_columns(box):
+    """The row copies of boxes without tensor copies, for every width from one
+    cell on: each chunk lies inside the row of the box, and each position that
+    is read holds the periodic column.  (The code of the kernels, built for the
+    host; the update kernel copies single floats through a table instead.)"""
+    L = lib()
+    out = np.empty(40, np.int32)
+    info = [ctypes.c_int() for _ in range(3)]
+    for nx in range(1, 81):
+        for W in (1, 2, 4):
+            if nx % W or (W == 1 and box > 0):
+                continue
+            for x0 in range(0, nx, 32):
+                inside = L.cellh_staged_columns(box, W, x0, nx, out.ctypes.data_as(ctypes.c_void_p),
+                                                *map(ctypes.byref, info))
+                assert inside == 1, (nx, W, x0)
+                origin, begin, end = (v.value for v in info)
+                assert begin + origin in (-2, -1, 0) and end + origin in (32, 33)
+                want = (x0 + origin + np.arange(begin, end)) % nx
+                assert np.array_equal(out[begin:end], want), (nx, W, x0)
