@@ -28,6 +28,7 @@
 
 #include "../../include/nmhd.h"
 #include "cell_flux_staged.cuh"
+#include "fields.h"
 #include "margin_ops.cuh"
 
 namespace nmhd {
@@ -743,18 +744,15 @@ int nmhd_batch_size(const nmhd_batch *b) { return b ? b->n : 0; }
 namespace {
 
 // Copies of one box's 8 fields into (to_box) or out of its current buffer,
-// whose parity the control block h says.
-nmhd_status box_copy(nmhd_batch *b, const StepCtl &h, int box, float *const *fields, int on_device, bool to_box) {
+// whose parity the control block h says.  held: one_run()'s, over one call.
+nmhd_status box_copy(nmhd_batch *b, const StepCtl &h, int box, float *const *fields, int on_device, bool to_box,
+                     nmhd::Allocation &held) {
   const BoxDesc &d = b->boxes[box];
   float *cur = h.parity ? d.w1 : d.w0;
   const size_t n = (size_t)d.g.n;
-  // fields that lie one after another, as on the device, are one copy: the
-  // copies of 256 boxes of 8.8k cells took 10 ms as 2,048 of 35 KB
-  bool together = true;
-  for (int v = 0; v < 8; ++v) {
+  for (int v = 0; v < 8; ++v)
     if (!fields[v]) return bfail(b, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
-    together = together && fields[v] == fields[0] + v * n;
-  }
+  const bool together = nmhd::one_run(fields, n, held, nmhd::allocation_of);
   const size_t bytes = sizeof(float) * n * (together ? 8 : 1);
   const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice
                                         : (to_box ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost);
@@ -771,8 +769,9 @@ nmhd_status set_states(nmhd_batch *b, int b0, int b1, const float *const *fields
   std::vector<StepCtl> h;
   nmhd_status st = read_ctls(b, h);
   if (st != NMHD_OK) return st;
+  nmhd::Allocation held = {};
   for (int box = b0; box < b1; ++box) {
-    st = box_copy(b, h[box], box, const_cast<float *const *>(fields + 8 * (box - b0)), on_device, true);
+    st = box_copy(b, h[box], box, const_cast<float *const *>(fields + 8 * (box - b0)), on_device, true, held);
     if (st != NMHD_OK) return st;
     h[box].status = 0;
     h[box].done = 0;
@@ -786,8 +785,9 @@ nmhd_status get_states(nmhd_batch *b, int b0, int b1, float *const *fields, int 
   std::vector<StepCtl> h;
   nmhd_status st = read_ctls(b, h);
   if (st != NMHD_OK) return st;
+  nmhd::Allocation held = {};
   for (int box = b0; box < b1; ++box) {
-    st = box_copy(b, h[box], box, fields + 8 * (box - b0), on_device, false);
+    st = box_copy(b, h[box], box, fields + 8 * (box - b0), on_device, false, held);
     if (st != NMHD_OK) return st;
   }
   BATCH_CUDA(b, cudaStreamSynchronize(b->stream));

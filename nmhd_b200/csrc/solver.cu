@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/nmhd.h"
+#include "fields.h"
 #include "mhd_math.cuh"
 #include "solver_impl.h"
 #include "step.cuh"
@@ -236,13 +237,13 @@ void drop_graphs(nmhd_solver *s) {
 nmhd_status copy_fields(nmhd_solver *s, float *dev_base, const float *const in[8], float *const out[8],
                         int on_device) {
   const size_t n = (size_t)s->g.n;
-  // fields that lie one after another, as on the device, are one copy
-  bool together = true;
+  const float *f[8];
   for (int v = 0; v < 8; ++v) {
-    const float *p = in ? in[v] : out[v], *first = in ? in[0] : out[0];
-    if (!p) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
-    together = together && p == first + v * n;
+    f[v] = in ? in[v] : out[v];
+    if (!f[v]) return fail(s, NMHD_ERR_INVALID_ARGUMENT, "field pointer is NULL");
   }
+  nmhd::Allocation held = {};
+  const bool together = nmhd::one_run(f, n, held, nmhd::allocation_of);
   const size_t bytes = sizeof(float) * n * (together ? 8 : 1);
   for (int v = 0; v < (together ? 1 : 8); ++v) {
     if (in)

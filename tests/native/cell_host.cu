@@ -6,6 +6,7 @@
 // results are the device's and the tests can compare them bitwise with the
 // oracle on a CPU.  Not part of the library; nothing in nmhd_b200 loads it.
 #include "../../nmhd_b200/csrc/cell_flux_staged.cuh"
+#include "../../nmhd_b200/csrc/fields.h"
 
 extern "C" {
 
@@ -91,4 +92,19 @@ extern "C" int cellh_staged_columns(int box, int W, int x0, int nx, int *out, in
     case 4: return copied_box<epi::ZYF>(W, x0, nx, out, origin, begin, end);
     default: return -1;
   }
+}
+
+// one_run() over a made-up address space: m allocations [begin[i], end[i]), the
+// rest pageable, or unknown to the driver.
+extern "C" int cellh_one_run(const uintptr_t *fields, long n, const uintptr_t *begin, const uintptr_t *end, int m,
+                             int known) {
+  const float *f[8];
+  for (int v = 0; v < 8; ++v) f[v] = reinterpret_cast<const float *>(fields[v]);
+  nmhd::Allocation held = {};
+  return nmhd::one_run(f, (size_t)n, held, [&](const void *p) {
+    nmhd::Allocation a = {known != 0, 0, 0};
+    for (int i = 0; i < m; ++i)
+      if (begin[i] <= (uintptr_t)p && (uintptr_t)p < end[i]) a.begin = begin[i], a.end = end[i];
+    return a;
+  });
 }
