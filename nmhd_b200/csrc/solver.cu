@@ -153,13 +153,27 @@ nmhd_status read_ctl(nmhd_solver *s, StepCtl &h) {
 __global__ void k_write_ctl(StepCtl *ctl, StepCtl h) { *ctl = h; }
 
 // In the stream's order, without waiting: the values travel as the kernel's
-// parameter.
+// parameter.  A kernel is launched on the current device's streams only, and the
+// calling thread may have another one current.
 nmhd_status write_ctl(nmhd_solver *s, const StepCtl &h) {
   s->ctl_known = false;
+  int current = s->device;
+  NMHD_CUDA(s, cudaGetDevice(&current));
+  if (current != s->device) NMHD_CUDA(s, cudaSetDevice(s->device));
   k_write_ctl<<<1, 1, 0, s->stream>>>(s->ctl, h);
-  NMHD_CUDA(s, cudaGetLastError());
+  const cudaError_t launched = cudaGetLastError();
+  if (current != s->device) NMHD_CUDA(s, cudaSetDevice(current));
+  NMHD_CUDA(s, launched);
   s->mirror = h;
   s->ctl_known = true;
+  return NMHD_OK;
+}
+
+// The same for the calls that return when the device has taken the values.
+nmhd_status write_ctl_and_wait(nmhd_solver *s, const StepCtl &h) {
+  const nmhd_status st = write_ctl(s, h);
+  if (st != NMHD_OK) return st;
+  NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
   return NMHD_OK;
 }
 
@@ -234,6 +248,7 @@ void drop_graphs(nmhd_solver *s) {
   s->graphs.clear();
 }
 
+// Enqueues the copies.
 nmhd_status copy_fields(nmhd_solver *s, float *dev_base, const float *const in[8], float *const out[8],
                         int on_device) {
   const size_t n = (size_t)s->g.n;
@@ -253,7 +268,6 @@ nmhd_status copy_fields(nmhd_solver *s, float *dev_base, const float *const in[8
       NMHD_CUDA(s, cudaMemcpyAsync(out[v], dev_base + v * n, bytes,
                                    on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s->stream));
   }
-  NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
   return NMHD_OK;
 }
 
@@ -304,7 +318,7 @@ nmhd_status nmhd_create(const nmhd_config *cfg, nmhd_solver **out) {
   h.cfl_cur = h.cfl_next = 0x7f800000u;
   h.goal = INFINITY;
   h.hist_cap = nmhd::kDtHistCap;
-  st = write_ctl(s, h);
+  st = write_ctl_and_wait(s, h);
   if (st != NMHD_OK) {
     g_create_error = s->err;
     nmhd_destroy(s);
@@ -348,7 +362,7 @@ nmhd_status nmhd_set_state(nmhd_solver *s, const float *const fields[8], int on_
   h.done = 0;
   h.cfl_cur = h.cfl_next = 0x7f800000u;
   s->cfl_ready = false;
-  return write_ctl(s, h);
+  return write_ctl_and_wait(s, h);
 }
 
 nmhd_status nmhd_get_state(nmhd_solver *s, float *const fields[8], int on_device) {
@@ -356,7 +370,10 @@ nmhd_status nmhd_get_state(nmhd_solver *s, float *const fields[8], int on_device
   StepCtl h;
   nmhd_status st = read_ctl(s, h);
   if (st != NMHD_OK) return st;
-  return copy_fields(s, current_buffer(s, h), nullptr, fields, on_device);
+  st = copy_fields(s, current_buffer(s, h), nullptr, fields, on_device);
+  if (st != NMHD_OK) return st;
+  NMHD_CUDA(s, cudaStreamSynchronize(s->stream));
+  return NMHD_OK;
 }
 
 nmhd_status nmhd_read(nmhd_solver *s, const char *path) {
@@ -520,7 +537,7 @@ nmhd_status nmhd_set_time(nmhd_solver *s, double current_time, int64_t generatio
   h.generation = generation;
   // The shearing fill depends on the time: recompute margins and CFL.
   s->cfl_ready = false;
-  return write_ctl(s, h);
+  return write_ctl_and_wait(s, h);
 }
 
 int64_t nmhd_dt_history(const nmhd_solver *s, float *out, int64_t n) {
@@ -896,7 +913,7 @@ nmhd_status nmhd_slab_begin(nmhd_solver *s, double goal_time) {
     h.cfl_cur = h.cfl_next = 0x7f800000u;
     h.blocks_done = 0;
   }
-  return write_ctl(s, h);
+  return write_ctl_and_wait(s, h);
 }
 
 nmhd_status nmhd_halo_pack(nmhd_solver *s, float *send_inc, float *send_dec) {
