@@ -341,10 +341,16 @@ __device__ __forceinline__ bool face_b_with(Smem &s, const GridParams &g, int a,
     hb = new_bx<kPow2>(q, s, g, W[hr], 32, lane & 3, lane >> 2, dt);
   }
   const int ix = fBX + BXs::at(a, b, c), iy = fBY + BYs::at(a, b, c), iz = fBZ + BZs::at(a, b, c);
-  F[ix] = new_bx<kPow2>(q, s, g, W[ix], a, b, c, dt);
-  F[iy] = new_by<kPow2>(q, s, g, W[iy], a, b, c, dt);
-  F[iz] = new_bz<kPow2>(q, s, g, W[iz], a, b, c, dt);
+  const float bx = new_bx<kPow2>(q, s, g, W[ix], a, b, c, dt);
+  const float by = new_by<kPow2>(q, s, g, W[iy], a, b, c, dt);
+  const float bz = new_bz<kPow2>(q, s, g, W[iz], a, b, c, dt);
+  F[ix] = bx;
+  F[iy] = by;
+  F[iz] = bz;
   if (hr >= 0) F[hr] = hb;
+  // a quotient by a numerator that is not finite, or that overflows, gives NaN
+  // in the one arithmetic and infinity in the other
+  q.positive(q.finite(bx, by, bz, hb));
   return q.hold();
 }
 
@@ -425,6 +431,7 @@ __device__ __forceinline__ bool finish_cell_with(const Smem &s, const GridParams
   const float eint = ene - q.div(0.5f * (mx * mx + my * my + mz * mz), drho) -
                      0.25f * (bx0 * bx0 + bx1 * bx1 + by0 * by0 + by1 * by1 + bz0 * bz0 + bz1 * bz1);
   const float po = eint * gm1;
+  q.positive(q.finite(vxo, vyo, vzo, po));  // as in face_b_with()
   if (g.shear) {
     const float ax = -2.0f * g.omega * vyo;
     const float ay = 2.0f * g.omega * vxo + 2.0f * g.q * (g.omega * g.omega) * (g.corner_y + g.dy * ((float)y + 0.5f));

@@ -162,11 +162,11 @@ __device__ __forceinline__ bool stage(Smem &s, const GridParams &g, const FluxMa
 // The states on either side of a face from the cells' values x0..x3, and from
 // sums of two values, which halve exactly where q.slope() holds.
 template <class Q>
-__device__ __forceinline__ void face_states(Q &q, const float x[4], float &l, float &r) {
+__host__ __device__ __forceinline__ void face_states(Q &q, const float x[4], float &l, float &r) {
   reconstruct4_with(q, x[0], x[1], x[2], x[3], l, r);
 }
 template <class Q>
-__device__ __forceinline__ void face_means(Q &q, const float s[4], float &l, float &r) {
+__host__ __device__ __forceinline__ void face_means(Q &q, const float s[4], float &l, float &r) {
   reconstruct4_with(q, s[0], s[1], s[2], s[3], l, r);
   l *= 0.5f;
   r *= 0.5f;

@@ -36,24 +36,28 @@ __host__ __device__ __forceinline__ void reconstruct4(float x0, float x1, float 
   right = x2 - d2 / 2.0f;
 }
 
-// The same reconstruction for slopes that are 0 or at least 2^-74 (q.slope()).
+// The same reconstruction for slopes that are 0 or at least 2^-73 (q.slope()).
 // The limited slope is the smaller magnitude where both
 // differences have one sign, else 0: min.xorsign.abs gives the smaller
 // magnitude, positive where the signs agree, so a maximum with 0 and a sign
 // copy replace a product, two comparisons and two selections.  The product of
 // two slopes that small would underflow to 0 and switch the limiter off, which
 // is why they are left to reconstruct4(); halving a slope that is not is
-// exact, so the half slope is added in one fused multiply-add.
+// exact, so the half slope is added in one fused multiply-add.  The bound holds
+// for the slopes of sums of two values too, which are twice those of their
+// means.  A NaN among the four cells gives a NaN state, whatever reconstruct4()
+// would select; the caller has to look for it.
 template <class A>
 __host__ __device__ __forceinline__ float limited_slope(A &q, float a, float b) {
 #ifdef __CUDA_ARCH__
   float t;
-  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(t) : "f"(a), "f"(b));
+  asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(t) : "f"(a), "f"(b));
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(t) : "f"(t));
 #else
   const float m = fabsf(a) < fabsf(b) ? fabsf(a) : fabsf(b);
-  float t = (float_bits(a) ^ float_bits(b)) >> 31 ? -m : m;
+  float t = fmaxf((float_bits(a) ^ float_bits(b)) >> 31 ? -m : m, 0.0f);
+  if (a != a || b != b) t = a + b;
 #endif
-  t = fmaxf(t, 0.0f);
   q.slope(t);
   return copysignf(t, b);
 }
@@ -320,7 +324,7 @@ __host__ __device__ __forceinline__ bool hlld_flux_with(A &q, const float gamma,
   const float SMn = sRv * (s.dr * s.ur) - sLv * (s.dl * s.ul) - pT_R + pT_L;
   const float pTn = dsR * pT_L - dsL * pT_R + s.dl * s.dr * sRv * sLv * (s.ur - s.ul);
   const Denominator dden = q.under(den);
-  const float S_M = q.div_bounded(SMn, dden), pT_s = q.div_bounded(pTn, dden);
+  const float S_M = q.div_bounded(SMn, dden, q.finite(s.vl, s.vr, s.wl, s.wr)), pT_s = q.div_bounded(pTn, dden);
 
   // The side of the contact that x/t = 0 lies on.  The operands are ordered
   // numbers here (a NaN fails the ranges), so of the fan's conditions only

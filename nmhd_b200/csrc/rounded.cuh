@@ -21,7 +21,7 @@
 // Square root of x: from y ~ 1/sqrt(x), g = x y is corrected by y/2 times the
 // exact residual x - g^2 (Markstein, same paper).
 //
-// Ranges: |b| in [2^-40, 2^31], a = 0 or |a| >= 2^-74, |a/b| < 2^127, x in
+// Ranges: |b| in [2^-40, 2^31], a = 0 or |a| >= 2^-73, |a/b| < 2^127, x in
 // [2^-90, 2^90]; no intermediate then overflows, and no residual loses bits to
 // underflow.  A zero quotient may come back as +0 where it is -0.
 #pragma once
@@ -92,11 +92,11 @@ __host__ __device__ __forceinline__ unsigned float_bits(float v) {
 // Whether the operands seen so far lie in the ranges above, kept as extremes
 // of their bit patterns.  positive(): in [2^-40, 2^24], as the largest distance
 // above the lower bound (unsigned: smaller, negative and NaN values wrap or lie
-// far above).  tiny(): 0 or at least 2^-74, as the least pattern less one (0
+// far above).  tiny(): 0 or at least 2^-73, as the least pattern less one (0
 // becomes the largest).  Two accumulators and one instruction a value: more of
 // either cost the Riemann solver spills.
 struct Ranges {
-  static constexpr unsigned kLow = (127u - 40u) << 23, kHigh = (127u + 24u) << 23, kTiny = (127u - 74u) << 23;
+  static constexpr unsigned kLow = (127u - 40u) << 23, kHigh = (127u + 24u) << 23, kTiny = (127u - 73u) << 23;
   unsigned far = 0u, least = 0xffffffffu;
   __host__ __device__ __forceinline__ void positive(float v) {
     const unsigned u = float_bits(v) - kLow;
@@ -125,10 +125,14 @@ struct Ranged {
     r.tiny(fabsf(a));
     return quotient(a, d);
   }
-  __host__ __device__ __forceinline__ float div_bounded(float a, const Denominator &d) {
+  __host__ __device__ __forceinline__ float div_bounded(float a, const Denominator &d, float least = 0x1p-40f) {
     // |a| 2^-36 + 2^-40 <= 2^24
-    r.positive(fmaf(fabsf(a), 0x1p-36f, 0x1p-40f));
+    r.positive(fmaf(fabsf(a), 0x1p-36f, least));
     return div(a, d);
+  }
+  // 2^-40 if all are finite, else NaN, which is in no range.
+  __host__ __device__ __forceinline__ static float finite(float a, float b, float c, float d) {
+    return fmaf(a, 0.0f, fmaf(b, 0.0f, fmaf(c, 0.0f, fmaf(d, 0.0f, 0x1p-40f))));
   }
   __host__ __device__ __forceinline__ static float root(float x) { return nmhd::root(x); }
   __host__ __device__ __forceinline__ bool hold() const { return r.hold(); }
@@ -141,7 +145,8 @@ struct Ieee {
   __host__ __device__ __forceinline__ static Denominator under(float b) { return Denominator{b, 0.0f}; }
   __host__ __device__ __forceinline__ static float ratio(float a, const Denominator &d) { return a / d.b; }
   __host__ __device__ __forceinline__ static float div(float a, const Denominator &d) { return a / d.b; }
-  __host__ __device__ __forceinline__ static float div_bounded(float a, const Denominator &d) { return a / d.b; }
+  __host__ __device__ __forceinline__ static float div_bounded(float a, const Denominator &d, float = 0.0f) { return a / d.b; }
+  __host__ __device__ __forceinline__ static float finite(float, float, float, float) { return 1.0f; }
   __host__ __device__ __forceinline__ static float root(float x) { return sqrtf(x); }
   __host__ __device__ __forceinline__ static bool hold() { return true; }
 };

@@ -108,3 +108,41 @@ extern "C" int cellh_one_run(const uintptr_t *fields, long n, const uintptr_t *b
     return a;
   });
 }
+
+// A face's flux from the four cells of its stencil: x holds 4 x (rho, u, v, w, p, By
+// sum, Bz sum), the last two sums of two face values; by hlld_flux_ranged() on the
+// states of reconstruct4_with() (ok[i]: whether it takes them) and by the plain
+// arithmetic on the means.
+extern "C" void cellh_face_f32(float gamma, const float *bx, const float *x, float *ranged, float *plain, int *ok,
+                               long n) {
+  const nmhd::Denominator gm1 = nmhd::denominator(gamma - 1.0f);
+  for (long i = 0; i < n; ++i) {
+    const float *c = x + 28 * i;
+    nmhd::HlldIn a, b;
+    nmhd::Ranged q;
+    nmhd::Ieee unchecked;
+    float *pa = &a.dl, *pb = &b.dl;
+    for (int v = 0; v < 7; ++v) {
+      const float y[4] = {c[v], c[7 + v], c[14 + v], c[21 + v]};
+      if (v == 0 || v == 4) nmhd::cell::sfx::face_states(unchecked, y, pa[2 * v], pa[2 * v + 1]);
+      else if (v < 5) nmhd::cell::sfx::face_states(q, y, pa[2 * v], pa[2 * v + 1]);
+      else nmhd::cell::sfx::face_means(q, y, pa[2 * v], pa[2 * v + 1]);
+      const float h = v < 5 ? 1.0f : 0.5f;
+      nmhd::reconstruct4(h * y[0], h * y[1], h * y[2], h * y[3], pb[2 * v], pb[2 * v + 1]);
+    }
+    ok[i] = nmhd::hlld_flux_with(q, gamma, gm1, bx[i], a, [&](int k, float v) { ranged[7 * i + k] = v; });
+    nmhd::hlld_flux_plain(gamma, bx[i], b, plain + 7 * i);
+  }
+}
+
+// face_means() alone, and reconstruct4() of the means.
+extern "C" void cellh_means_f32(const float *sums, float *ranged, float *plain, int *ok, long n) {
+  for (long i = 0; i < n; ++i) {
+    const float *s = sums + 4 * i;
+    nmhd::Ranged q;
+    nmhd::cell::sfx::face_means(q, s, ranged[2 * i], ranged[2 * i + 1]);
+    q.positive(1.0f);
+    ok[i] = q.hold();
+    nmhd::reconstruct4(0.5f * s[0], 0.5f * s[1], 0.5f * s[2], 0.5f * s[3], plain[2 * i], plain[2 * i + 1]);
+  }
+}

@@ -37,6 +37,8 @@ def lib():
         L.cellh_hlld_many_f32.argtypes = [ctypes.c_float, P, P, P, ctypes.c_long]
         L.cellh_reconstruct_f32.argtypes = [P, P, ctypes.c_long]
         L.cellh_reconstruct_ranged_f32.argtypes = [P, P, P, ctypes.c_long]
+        L.cellh_means_f32.argtypes = [P, P, P, P, ctypes.c_long]
+        L.cellh_face_f32.argtypes = [ctypes.c_float, P, P, P, P, P, ctypes.c_long]
         L.cellh_hlld_ranged_f32.argtypes = [ctypes.c_float, P, P, P, P, P, ctypes.c_long]
         _lib = L
     return _lib
@@ -135,7 +137,7 @@ def test_device_reconstruction_is_the_minbee_limiter():
 def test_ranged_reconstruction_is_the_plain_one_where_it_takes_the_slopes(scale):
     """reconstruct4_with against reconstruct4 (equal values; the sign of a zero
     may differ), on slopes of order `scale` on a zero and on a non-zero mean:
-    taken unless a non-zero slope is below 2^-74."""
+    taken unless a non-zero slope is below 2^-73."""
     rng = np.random.default_rng(13)
     n = 40000
     x = (rng.normal(0.0, 1.0, (n, 4)) * scale).astype(np.float32)
@@ -150,3 +152,45 @@ def test_ranged_reconstruction_is_the_plain_one_where_it_takes_the_slopes(scale)
     assert np.array_equal(lr[took], ref[took])
     assert took[::3].all() or scale == 1.0
     assert took.mean() > 0.95 if scale > 1e-21 else not took[1::3].all()
+
+
+def assert_face_takes_only_what_it_computes_alike(bx, x):
+    n = len(bx)
+    a, b, ok = np.empty((n, 7), np.float32), np.empty((n, 7), np.float32), np.empty(n, np.int32)
+    lib().cellh_face_f32(5.0 / 3.0, bx.ctypes.data, x.ctypes.data, a.ctypes.data, b.ctypes.data, ok.ctypes.data, n)
+    took = ok != 0
+    assert np.array_equal(a[took], b[took], equal_nan=True)
+
+
+def face_cells(rng, n):
+    """Four cells a face: density, velocities (some supersonic), pressure, sums of B."""
+    x = rng.normal(0.0, 1.0, (n, 4, 7))
+    x[:, :, 0] = rng.uniform(0.5, 2.0, (n, 4))
+    x[:, :, 4] = rng.uniform(0.1, 2.0, (n, 4))
+    x[:, :, 1] += rng.choice([0.0, 6.0, -6.0], (n, 1))
+    return rng.normal(0.0, 0.5, n).astype(np.float32), x.astype(np.float32)
+
+
+@pytest.mark.parametrize("value", [np.nan, -np.nan, np.inf, -np.inf])
+def test_ranged_face_leaves_cells_that_are_not_finite_to_the_plain_one(value):
+    """One value of one of a face's four cells is not finite: its flux by the shared
+    reciprocals is the plain one, NaN for NaN, or is not taken."""
+    rng = np.random.default_rng(17)
+    n = 56000
+    bx, x = face_cells(rng, n)
+    at = np.arange(n)
+    x[at, at % 4, at // 4 % 7] = np.float32(value)
+    assert_face_takes_only_what_it_computes_alike(bx, np.ascontiguousarray(x))
+
+
+def test_ranged_means_with_slopes_at_the_limiters_underflow():
+    """Sums of two values with differences of a few 2^-75: the products of the means'
+    slopes underflow to 0 below 2^-75, and the plain limiter is then off."""
+    rng = np.random.default_rng(19)
+    n = 40000
+    s = (rng.integers(-24, 25, (n, 4)) * 2.0 ** -75).astype(np.float32)
+    a, b, ok = np.empty((n, 2), np.float32), np.empty((n, 2), np.float32), np.empty(n, np.int32)
+    lib().cellh_means_f32(s.ctypes.data, a.ctypes.data, b.ctypes.data, ok.ctypes.data, ctypes.c_long(n))
+    took = ok != 0
+    assert 0.05 < took.mean() < 0.95
+    assert np.array_equal(a[took], b[took])

@@ -36,3 +36,27 @@ def test_staged_paths_match_oracle(gpu, nx, ny, nz, units):
     assert np.isfinite(o["state"]).all()
     assert r["time"] == o["time"]
     assert_same(r["state"], o["state"])
+
+
+@pytest.mark.parametrize("n", [(24, 20, 12), (32, 16, 8)])  # spacings that are no powers of two, and that are
+@pytest.mark.parametrize("value", [np.nan, np.inf, -3e38])
+@pytest.mark.parametrize("time_order", [1, 2])
+def test_states_that_are_not_finite_spread_as_in_the_per_cell_kernels(gpu, n, value, time_order):
+    """One value of one cell is not finite or overflows: the step ends in an error,
+    and what it leaves is the per-cell kernels' state (the compiler's quotients and
+    the plain limiter), NaN for NaN and infinity for infinity."""
+    from nmhd_b200._lib import NmhdError
+    from nmhd_b200.solver import MHDSolver
+    for field in range(8):
+        cfg, s = orszag_tang_3d(n[0], ny=n[1], nz=n[2])
+        cfg.time_order = time_order
+        s[field, 5, 9, 11] = value
+        found = []
+        for variant in (2, 5):
+            with MHDSolver(cfg) as sol:
+                sol.set_kernel(variant)
+                sol.set_state(s)
+                with pytest.raises(NmhdError):
+                    sol.step(1)
+                found.append(sol.get_state())
+        assert np.array_equal(*found, equal_nan=True), (field, int((found[0] != found[1]).sum()))
