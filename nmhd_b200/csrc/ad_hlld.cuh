@@ -651,7 +651,9 @@ static __device__ __noinline__ HAdjoint hlld_adjoint_of_type(float gamma, float 
 }
 static __device__ __forceinline__ void hlld_adjoint_ranged(const float gamma, const float Bx, const HState<float> &in,
                                                            const float lf[7], HState<float> &ls, float &lBx) {
-  if (hlld_adjoint_with<OfRanges>(gamma, Bx, in, lf, ls, lBx) && denominator_in_range(gamma - 1.0f)) return;
+  if (denominator_in_range(gamma - 1.0f) && likely_in_range(in.dl, in.pl, Bx, in.byl, in.bzl) &&
+      hlld_adjoint_with<OfRanges>(gamma, Bx, in, lf, ls, lBx))
+    return;
   const HAdjoint o = hlld_adjoint_of_type(gamma, Bx, in, lf[0], lf[1], lf[2], lf[3], lf[4], lf[5], lf[6]);
   ls = o.s;
   lBx = o.bx;

@@ -359,7 +359,7 @@ __device__ __forceinline__ void face_b(Smem &s, const GridParams &g, int a, int 
                                        float dt) {
   if (kPow2) {
     face_b_with<true, Ieee>(s, g, a, b, c, warp, lane, dt);
-  } else if (!(face_b_with<false, Ranged>(s, g, a, b, c, warp, lane, dt) && g.ranged)) {
+  } else if (!(g.ranged && face_b_with<false, Ranged>(s, g, a, b, c, warp, lane, dt))) {
     face_b_with<false, Ieee>(s, g, a, b, c, warp, lane, dt);
   }
 }
@@ -474,7 +474,7 @@ __device__ __forceinline__ void finish_cell(const Smem &s, const GridParams &g, 
   // tests then cost what they save (1156 against 1147 warp instructions a
   // stage, and a second copy of the code).
   if (!kPow2) {
-    if (finish_cell_with<kPow2, kFinal, Ranged>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed) && g.ranged)
+    if (g.ranged && finish_cell_with<kPow2, kFinal, Ranged>(s, g, wb, wo, flux, a, b, c, x, y, z, dt, bad, speed))
       return;
     // The compiler's division, on inputs read again (the opaque coordinate
     // keeps the first reading's values from being held in registers).

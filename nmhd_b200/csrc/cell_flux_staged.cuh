@@ -246,18 +246,21 @@ __device__ __forceinline__ HlldIn staged_input(Q &q, const GridParams &g, bool o
   return in;
 }
 
-// The lower ax-face of cell ci in the plain arithmetic: a call, so that its
-// registers and code stay out of the loop that seldom needs it.
-static __device__ __noinline__ void plain_face(const GridParams &g, const float *w, float *flux, int ci, int ax, int o,
-                                               int yidx, float half_dt) {
-  const int sa = ax == 0 ? 1 : ax == 1 ? DY : DZ;
-  const int t1 = ax == 0 ? DY : ax == 1 ? DZ : 1, t2 = ax == 0 ? DZ : ax == 1 ? 1 : DY;
-  float f[7];
-  hlld_flux_plain(g.gamma, w[(5 + ax) * FS + ci],
-                  face_input<SharedLd>(g, w, FS, ci, ax, -2 * sa, -sa, sa, t1, t2, yidx, 2.0f * half_dt), f);
-  float *out = flux + (size_t)(7 * ax) * g.n + o;
+// The lower faces along axes ax0..ax1-1 of cell ci in the plain arithmetic: a call,
+// so that its registers and code stay out of the loop that seldom needs it.
+static __device__ __noinline__ void plain_faces(const GridParams &g, const float *w, float *flux, int ci, int ax0,
+                                                int ax1, int o, int yidx, float half_dt) {
+#pragma unroll 1
+  for (int ax = ax0; ax < ax1; ++ax) {
+    const int sa = ax == 0 ? 1 : ax == 1 ? DY : DZ;
+    const int t1 = ax == 0 ? DY : ax == 1 ? DZ : 1, t2 = ax == 0 ? DZ : ax == 1 ? 1 : DY;
+    float f[7];
+    hlld_flux_plain(g.gamma, w[(5 + ax) * FS + ci],
+                    face_input<SharedLd>(g, w, FS, ci, ax, -2 * sa, -sa, sa, t1, t2, yidx, 2.0f * half_dt), f);
+    float *out = flux + (size_t)(7 * ax) * g.n + o;
 #pragma unroll
-  for (int k = 0; k < 7; ++k) out[(size_t)k * g.n] = f[k];
+    for (int k = 0; k < 7; ++k) out[(size_t)k * g.n] = f[k];
+  }
 }
 
 // The lower-face fluxes along axes ax0..ax1-1 of tile-local cell (a, b, c) at
@@ -274,29 +277,39 @@ __device__ __forceinline__ void flux_cell_order(const GridParams &g, bool order2
                                                 unsigned o, int y, float dt, int ax0, int ax1) {
   const size_t N = (size_t)g.n;
   const float half_dt = 0.5f * dt;
+#if !NMHD_FAST_ARITH
+  const bool ranged = g.gm1_ranged &&
+                      likely_in_range(w[ci], w[4 * FS + ci], w[5 * FS + ci], w[6 * FS + ci], w[7 * FS + ci]);
+#endif
 #pragma unroll 1
   for (int ax = ax0; ax < ax1; ++ax) {
     // field k: uniform base, 32-bit byte offset of the cell (at most 2^28 cells)
     char *base = reinterpret_cast<char *>(flux + (size_t)(7 * ax) * N);
     auto out = [&](int k, float v) { *reinterpret_cast<float *>(base + k * (4 * N) + 4u * o) = v; };
+    const float bn = w[(5 + ax) * FS + ci];
+    auto input = [&](auto &q) {
+      return ax == 0   ? staged_input<0>(q, g, order2, w, ci, y, half_dt)
+             : ax == 1 ? staged_input<1>(q, g, order2, w, ci, y, half_dt)
+                       : staged_input<2>(q, g, order2, w, ci, y, half_dt);
+    };
 #if NMHD_FAST_ARITH
     AsCompiled q;
-#else
-    Ranged q;
-#endif
-    const float bn = w[(5 + ax) * FS + ci];
-    HlldIn in;
-    if (ax == 0) in = staged_input<0>(q, g, order2, w, ci, y, half_dt);
-    else if (ax == 1) in = staged_input<1>(q, g, order2, w, ci, y, half_dt);
-    else in = staged_input<2>(q, g, order2, w, ci, y, half_dt);
-#if NMHD_FAST_ARITH
     float f[7];
-    hlld_flux_plain(g.gamma, bn, in, f);
+    hlld_flux_plain(g.gamma, bn, input(q), f);
 #pragma unroll
     for (int k = 0; k < 7; ++k) out(k, f[k]);
 #else
-    const bool ok = hlld_flux_with(q, g.gamma, g.gm1, bn, in, out);
-    if (!(ok && g.ranged)) plain_face(g, w, flux, ci, ax, (int)o, y, half_dt);
+    bool ok = false;
+    if (ranged) {
+      Ranged q;
+      const HlldIn in = input(q);
+      ok = hlld_flux_with(q, g.gamma, g.gm1, bn, in, out);
+    }
+    if (!ok) {
+      // the cell's other faces too: where one is out of range they mostly are
+      plain_faces(g, w, flux, ci, ax, ax1, (int)o, y, half_dt);
+      return;
+    }
 #endif
   }
 }

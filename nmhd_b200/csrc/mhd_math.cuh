@@ -430,7 +430,9 @@ __host__ __device__ __forceinline__ bool hlld_flux_ranged(const float gamma, con
 }
 
 __host__ __device__ __forceinline__ void hlld_flux(const float gamma, const float Bx, const HlldIn &s, float f[7]) {
-  if (denominator_in_range(gamma - 1.0f) && hlld_flux_ranged(gamma, denominator(gamma - 1.0f), Bx, s, f)) return;
+  if (denominator_in_range(gamma - 1.0f) && likely_in_range(s.dl, s.pl, Bx, s.byl, s.bzl) &&
+      hlld_flux_ranged(gamma, denominator(gamma - 1.0f), Bx, s, f))
+    return;
   hlld_flux_plain(gamma, Bx, s, f);
 }
 

@@ -109,6 +109,19 @@ struct Ranges {
   __host__ __device__ __forceinline__ bool hold() const { return far <= kHigh - kLow && least >= kTiny - 1u; }
 };
 
+// Whether a cell's faces are likely to hold (known before they are solved): its
+// density and pressure are in the range of positive(), as its faces' must be, and
+// no field is so weak, without being 0, that products of two leave tiny()'s.
+__host__ __device__ __forceinline__ bool likely_in_range(float d, float p, float bx, float by, float bz) {
+  Ranges r;
+  r.positive(d);
+  r.positive(p);
+  r.tiny(fabsf(bx) * 0x1p-36f);  // |bx| >= 2^-37
+  r.tiny(fabsf(by) * 0x1p-36f);
+  r.tiny(fabsf(bz) * 0x1p-36f);
+  return r.hold();
+}
+
 // Arithmetic of code written once over its quotients and roots: div() checks
 // its numerator (div_bounded() also from above, by 2^60), ratio() and root()
 // leave their operands to positive(), and hold() says at the end whether every

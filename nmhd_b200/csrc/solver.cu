@@ -101,8 +101,9 @@ GridParams nmhd::derive_grid(const nmhd_config &c) {
   g.inv_dx = 1.0f / g.dx;
   g.inv_dy = 1.0f / g.dy;
   g.inv_dz = 1.0f / g.dz;
-  g.ranged = nmhd::denominator_in_range(gm1) && nmhd::denominator_in_range(g.dx) &&
-             nmhd::denominator_in_range(g.dy) && nmhd::denominator_in_range(g.dz);
+  g.gm1_ranged = nmhd::denominator_in_range(gm1);
+  g.ranged = g.gm1_ranged && nmhd::denominator_in_range(g.dx) && nmhd::denominator_in_range(g.dy) &&
+             nmhd::denominator_in_range(g.dz);
   return g;
 }
 

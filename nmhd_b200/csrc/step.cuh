@@ -28,7 +28,7 @@ struct GridParams {
   float inv_dx, inv_dy, inv_dz;
   int pow2_spacing;
   Denominator gm1;  // gamma - 1 as a denominator
-  int ranged;       // gamma - 1 and the spacings lie in the range of denominators (rounded.cuh)
+  int gm1_ranged, ranged;  // gamma - 1, and the spacings too, lie in the range of denominators (rounded.cuh)
 };
 
 // Device-resident step control.  The time step is a pure function of

@@ -7,7 +7,8 @@ operation rounded the same."""
 import numpy as np
 import pytest
 
-from nmhd_b200.problems import orszag_tang_3d
+from nmhd_b200.problems import orszag_tang_3d, shearing_box
+from nmhd_b200.solver import MHDSolver
 from oracle import oracle
 
 from test_parity_gpu import assert_same, run_gpu
@@ -60,3 +61,31 @@ def test_states_that_are_not_finite_spread_as_in_the_per_cell_kernels(gpu, n, va
                     sol.step(1)
                 found.append(sol.get_state())
         assert np.array_equal(*found, equal_nan=True), (field, int((found[0] != found[1]).sum()))
+
+
+@pytest.mark.parametrize("extent", [3e-13, 5e12])
+def test_spacings_out_of_range_match_oracle(gpu, extent):
+    """Spacings below 2^-40 and above 2^30, which only the update divides by."""
+    cfg, s = orszag_tang_3d(36, ny=14, nz=6, extent=extent)
+    o = oracle.proceed(cfg, s, 3)
+    r = run_gpu(cfg, s, 3)
+    assert np.isfinite(o["state"]).all()
+    assert r["time"] == o["time"]
+    assert_same(r["state"], o["state"])
+
+
+def test_faces_out_of_range_are_not_solved_twice(gpu):
+    """Density and pressure, or the field, in units that the shared reciprocals do
+    not cover: the faces take the plain arithmetic alone, 1.4 times the usual launch
+    and not 2.3."""
+    cfg, s = shearing_box(n_radial=64, n_azimuthal=128, n_vertical=64)
+    times = {}
+    for units, scale in (("usual", [1.0, 1.0]), ("light", [2.0 ** -46, 2.0 ** -23]), ("weak", [1.0, 1e-18])):
+        w = s.copy()
+        w[[0, 4]] *= np.float32(scale[0])
+        w[5:8] *= np.float32(scale[1])
+        with MHDSolver(cfg) as sol:
+            sol.set_state(w)
+            sol.step(4)
+            times[units] = min(sol.profile(4)["flux_stage1"][0] for _ in range(5))
+    assert times["light"] < 1.8 * times["usual"] and times["weak"] < 1.8 * times["usual"], times
