@@ -308,9 +308,8 @@ nmhd_status nmhd_batch_set_schedule(nmhd_batch *b, int kernel, int persistent, i
  * unchanged.  trials_out (may be NULL) receives up to max_trials rows of
  * (kernel, persistent, split, ms per launch), the two comparisons as rows
  * (4, persistent, staged, ms per flux launch) and (3, persistent, fused, ms
- * per stage update; with the passes on, only where a box's own tile is 32 x 4 x
- * 2).  Returns the number of rows written or a negative
- * nmhd_status.
+ * per stage update), with the passes on where they take a box.  Returns the
+ * number of rows written or a negative nmhd_status.
  * Every schedule gives bitwise the same result. */
 int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_trials);
 const char *nmhd_batch_last_error(const nmhd_batch *b);

@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kThreads, KIND == 0   ? NMHD_BATCH_MIN_BLOCKS_
 
 // Constrained transport and conserved update of the boxes of the staged passes
 // in one pass per tile: the single-box fused epilogue
-// (cell_epilogue.cuh, staging with cp.async), tiles [tb, te) of the staged list,
+// (cell_epilogue.cuh; tensor copies where the box has maps), tiles [tb, te) of the staged list,
 // persistent or one tile per CTA.
 #ifndef NMHD_BATCH_MIN_BLOCKS_EPI
 #define NMHD_BATCH_MIN_BLOCKS_EPI 5
@@ -255,9 +255,9 @@ __global__ void __launch_bounds__(kThreads, NMHD_BATCH_MIN_BLOCKS_EPI)
 }
 
 // Face fluxes of the boxes of the staged passes from a shared copy of each
-// tile's stencil: the single-box staged flux kernel (cell_flux_staged.cuh,
-// staging with cp.async), tiles [tb, te) of the group, persistent or one
-// tile per CTA.
+// tile's stencil: the single-box staged flux kernel (cell_flux_staged.cuh; tensor
+// copies where the box has maps), tiles [tb, te) of the staged list, persistent or
+// one tile per CTA.
 #ifndef NMHD_BATCH_MIN_BLOCKS_SFLUX
 #define NMHD_BATCH_MIN_BLOCKS_SFLUX 4
 #endif
@@ -1054,16 +1054,13 @@ int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_tri
     b->split[kind] = choice_split;
   }
   // The face fluxes with the chosen schedule against the staged flux pass for
-  // the 32 x 4 x 2 boxes (fluxes split), one tile per CTA or persistent:
+  // the boxes it takes (fluxes split), one tile per CTA or persistent:
   // rows (4, persistent, staged, ms per launch).
   {
     const bool keep_split = b->split[0];
     double best = 1e30;
-    bool best_on = false, best_p = false, any_fixed = false, any_staged = false;
-    for (const BatchGroup &p : b->groups) {
-      any_fixed = any_fixed || p.fixed_tiles > 0;
-      any_staged = any_staged || p.staged_tiles > 0;
-    }
+    bool best_on = false, best_p = false, any_staged = false;
+    for (const BatchGroup &p : b->groups) any_staged = any_staged || p.staged_tiles > 0;
     for (int trial = 0; trial < 3 && e == cudaSuccess; ++trial) {
       const int on = trial > 0, ps = trial == 2;
       if (on && !any_staged) break;
@@ -1079,7 +1076,7 @@ int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_tri
       if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
       if (e != cudaSuccess) break;
       const double per = ms / reps;
-      if (trials_out && written < max_trials && (!on || any_fixed)) {
+      if (trials_out && written < max_trials) {
         trials_out[4 * written + 0] = 4;
         trials_out[4 * written + 1] = ps;
         trials_out[4 * written + 2] = on;
@@ -1098,17 +1095,14 @@ int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_tri
     if (best_on) b->split[0] = true;
   }
   // The stage's update (constrained transport, then conserved update) with
-  // the chosen schedules, against the fused pass for the 32 x 4 x 2 boxes
-  // (both kernels split), one tile per CTA or persistent: rows of kernel 3,
+  // the chosen schedules, against the fused pass for the boxes of the staged
+  // passes (both kernels split), one tile per CTA or persistent: rows of kernel 3,
   // (3, persistent, fused, ms per update).
   {
     const bool keep_split[2] = {b->split[1], b->split[2]};
     double best = 1e30;
-    bool best_fuse = false, best_pf = false, any_fixed = false, any_staged = false;
-    for (const BatchGroup &p : b->groups) {
-      any_fixed = any_fixed || p.fixed_tiles > 0;
-      any_staged = any_staged || p.staged_tiles > 0;
-    }
+    bool best_fuse = false, best_pf = false, any_staged = false;
+    for (const BatchGroup &p : b->groups) any_staged = any_staged || p.staged_tiles > 0;
     for (int trial = 0; trial < 3 && e == cudaSuccess; ++trial) {
       const int f = trial > 0, pf = trial == 2;
       if (f && !any_staged) break;
@@ -1128,7 +1122,7 @@ int nmhd_batch_autotune(nmhd_batch *b, int reps, double *trials_out, int max_tri
       if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
       if (e != cudaSuccess) break;
       const double per = ms / reps;
-      if (trials_out && written < max_trials && (!f || any_fixed)) {
+      if (trials_out && written < max_trials) {
         trials_out[4 * written + 0] = 3;
         trials_out[4 * written + 1] = pf;
         trials_out[4 * written + 2] = f;
