@@ -268,7 +268,8 @@ static __device__ __noinline__ void plain_faces(const GridParams &g, const float
 // one Riemann solver (three overflow the instruction caches) and a branch per
 // axis that reads its input: with the axis a run-time number in the input too,
 // a tenth of the instructions made addresses.  256x128x64 box: 1,912 warp
-// instructions for a warp's three faces (2,293 before), 162 us a launch (181),
+// instructions for a warp's three faces (2,293 before), 162 us a launch (181; 154
+// now that the tiles at x edges are staged by tensor copies too),
 // 72 % of the issue slots filled.  Four CTAs/SM hide the start and the staging
 // of a tile better than one persistent CTA of 1,024 threads with a ring of five
 // copies (201 us: its spills miss the small L1 that is left) or a stagger of

@@ -16,8 +16,12 @@ from test_parity_gpu import assert_same, run_gpu
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("nx,ny,nz", [(1, 5, 3), (2, 13, 7), (3, 5, 3), (4, 13, 7), (6, 5, 3), (34, 13, 7), (35, 13, 7), (36, 13, 7), (37, 9, 5), (64, 16, 8), (70, 18, 6),
-                                      (100, 14, 6)])
+@pytest.mark.parametrize("nx,ny,nz", [(1, 5, 3), (2, 13, 7), (3, 5, 3), (4, 13, 7), (6, 5, 3), (34, 13, 7),
+                                      (35, 13, 7), (36, 13, 7), (37, 9, 5), (64, 16, 8), (70, 18, 6), (100, 14, 6),
+                                      # more tiles than SMs: a CTA takes a tile's three axes
+                                      (100, 34, 24), (102, 34, 24), (101, 34, 24),
+                                      # 1,105 tiles: the clock advances in a kernel of its own
+                                      (130, 50, 34)])
 @pytest.mark.parametrize("units", ["plain", "light", "light_mixed", "dense_mixed", "still"])
 def test_staged_paths_match_oracle(gpu, nx, ny, nz, units):
     cfg, s = orszag_tang_3d(nx, ny=ny, nz=nz)
