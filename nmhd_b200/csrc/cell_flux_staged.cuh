@@ -173,10 +173,11 @@ __host__ __device__ __forceinline__ void face_means(Q &q, const float s[4], floa
 }
 #if NMHD_FAST_ARITH
 // The fast-arithmetic kernel keeps face_input()'s and hlld_flux_plain()'s
-// operations as they stand.  With products by shared approximate reciprocals
-// and the three-instruction limiter a launch took 122 us instead of 141
-// (256x128x64 box), but after 16 steps the state was off the FP64 one by 5.3e-4
-// instead of 4.6e-4.
+// operations as they stand, so that runs of that mode keep their bits.  With
+// products by shared approximate reciprocals and the three-instruction limiter a
+// launch took 122 us instead of 141 (256x128x64 box): as near to an FP64 run (one
+// step of six boxes, five seeds each: the same error to three digits), but another
+// result, 4.7e-4 away after 16 steps.
 struct AsCompiled {};
 __device__ __forceinline__ void face_states(AsCompiled, const float x[4], float &l, float &r) {
   reconstruct4(x[0], x[1], x[2], x[3], l, r);
