@@ -275,8 +275,9 @@ static __device__ __noinline__ void plain_faces(const GridParams &g, const float
 // of a tile better than one persistent CTA of 1,024 threads with a ring of five
 // copies (201 us: its spills miss the small L1 that is left) or a stagger of
 // the first CTAs (172 us).
-__device__ __forceinline__ void flux_cell_order(const GridParams &g, bool order2, const float *w, float *__restrict__ flux, int ci,
-                                                unsigned o, int y, float dt, int ax0, int ax1) {
+__device__ __forceinline__ void flux_cell_order(const GridParams &g, bool order2, const float *w,
+                                                float *__restrict__ flux, int ci, unsigned o, int y, float dt, int ax0,
+                                                int ax1) {
   const size_t N = (size_t)g.n;
   const float half_dt = 0.5f * dt;
 #if !NMHD_FAST_ARITH

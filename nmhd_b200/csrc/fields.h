@@ -28,7 +28,7 @@ inline Allocation allocation_of(const void *p) {
                     q == cudaDriverEntryPointSuccess;
     return reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(ok ? fn : nullptr);
   }();
-  CUdeviceptr begin = 0;
+  CUdeviceptr begin = 0;  // both stay 0 for pageable memory
   size_t size = 0;
   CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
   void *to[2] = {&begin, &size};

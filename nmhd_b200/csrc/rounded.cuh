@@ -111,14 +111,12 @@ struct Ranges {
 
 // Whether a cell's faces are likely to hold (known before they are solved): its
 // density and pressure are in the range of positive(), as its faces' must be, and
-// no field is so weak, without being 0, that products of two leave tiny()'s.
+// its field is 0 or not so weak that products of two components leave tiny()'s.
 __host__ __device__ __forceinline__ bool likely_in_range(float d, float p, float bx, float by, float bz) {
   Ranges r;
   r.positive(d);
   r.positive(p);
-  r.tiny(fabsf(bx) * 0x1p-36f);  // |bx| >= 2^-37
-  r.tiny(fabsf(by) * 0x1p-36f);
-  r.tiny(fabsf(bz) * 0x1p-36f);
+  r.tiny(fmaxf(fmaxf(fabsf(bx), fabsf(by)), fabsf(bz)) * 0x1p-36f);  // 0 or at least 2^-37
   return r.hold();
 }
 

@@ -146,3 +146,7 @@ extern "C" void cellh_means_f32(const float *sums, float *ranged, float *plain, 
     nmhd::reconstruct4(0.5f * s[0], 0.5f * s[1], 0.5f * s[2], 0.5f * s[3], plain[2 * i], plain[2 * i + 1]);
   }
 }
+
+extern "C" int cellh_likely_in_range(float d, float p, float bx, float by, float bz) {
+  return nmhd::likely_in_range(d, p, bx, by, bz);
+}

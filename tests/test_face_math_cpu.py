@@ -194,3 +194,15 @@ def test_ranged_means_with_slopes_at_the_limiters_underflow():
     took = ok != 0
     assert 0.05 < took.mean() < 0.95
     assert np.array_equal(a[took], b[took])
+
+
+@pytest.mark.parametrize("cell, likely", [
+    ((1.0, 1.0, 0.0, 0.0, 0.0), True), ((1.0, 1.0, 1e-3, 0.0, 1e-9), True),
+    ((1.0, 1.0, 0.5, 1e-20, -1e-13), True),  # one strong component
+    ((1.0, 1.0, 1e-12, -1e-13, 0.0), False), ((1.0, 1.0, 0.0, 0.0, -1e-30), False),
+    ((2.0 ** -46, 1.0, 0.1, 0.1, 0.1), False), ((1.0, 2.0 ** 30, 0.1, 0.1, 0.1), False), ((1.0, -1.0, 0.1, 0.1, 0.1), False),
+    ((np.nan, 1.0, 0.1, 0.1, 0.1), False)])
+def test_cells_whose_faces_are_unlikely_to_hold(cell, likely):
+    f = lib().cellh_likely_in_range
+    f.argtypes = [ctypes.c_float] * 5
+    assert bool(f(*cell)) == likely
